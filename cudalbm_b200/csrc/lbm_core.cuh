@@ -202,40 +202,6 @@ __device__ __forceinline__ unsigned node_type(int x, int y, int z, int nx, int n
            (z == 0 ? BACK : 0u) | (z == nz - 1 ? FRONT : 0u);
 }
 
-// Bit q set if direction q has the given sign along the given axis.
-template <int AXIS, int SIGN>
-__host__ __device__ constexpr unsigned dir_mask()
-{
-    unsigned m = 0;
-    for (int q = 0; q < 27; q++) {
-        const int c = AXIS == 0 ? cx_of(q) : (AXIS == 1 ? cy_of(q) : cz_of(q));
-        if (c == SIGN)
-            m |= 1u << q;
-    }
-    return m;
-}
-
-// Directions that stream into a node of class t from outside the domain
-// (the complement of incomingSwitch, velocitySet.cuh:204-220).
-__device__ __forceinline__ unsigned unknown_dirs(unsigned t)
-{
-    return ((t & EAST) ? dir_mask<0, -1>() : 0u) | ((t & WEST) ? dir_mask<0, 1>() : 0u) |
-           ((t & NORTH) ? dir_mask<1, -1>() : 0u) | ((t & SOUTH) ? dir_mask<1, 1>() : 0u) |
-           ((t & FRONT) ? dir_mask<2, -1>() : 0u) | ((t & BACK) ? dir_mask<2, 1>() : 0u);
-}
-
-// The reference sums incomingSwitch*f_q with incomingSwitch in {0, 1}.  A zero
-// term leaves a right fold's value unchanged, so zeroing the unknown f_q and
-// folding as for an interior node gives the same bits as the masked sums.
-template <int Q, int q = 0>
-__device__ __forceinline__ void zero_unknown(float *f, unsigned unknown)
-{
-    if constexpr (q < Q) {
-        f[q] = ((unknown >> q) & 1u) ? 0.0f : f[q];
-        zero_unknown<Q, q + 1>(f, unknown);
-    }
-}
-
 // The ten raw sums the moments are built from: sum f, sum f c_a, sum f c_a c_b.
 template <int Q>
 __device__ __forceinline__ void moment_folds(const float *f, float *s)
@@ -511,14 +477,15 @@ __device__ __forceinline__ void scale_collide(float *m, const Relax &rx)
     m[8] = rx.t_omega * m[8] + om * (m[2]) * (m[3]);
 }
 
-// Full node update from the streamed populations f[Q] (in direction order).
+// Full node update from the streamed populations f[Q] (in direction order;
+// those that come from outside the mesh are zero, so that the folds of a
+// boundary node are the sums over its known populations: the reference sums
+// incomingSwitch * f_q with incomingSwitch in {0, 1}, velocitySet.cuh:204-220,
+// and a zero term leaves a right fold's value unchanged).
 // Returns the stored (post-collision) moments with rho still including rho0.
-// f is clobbered (unknown directions of boundary nodes are zeroed).
 template <int Q, int SCI = 1>
-__device__ __forceinline__ void node_update(float *f, unsigned type, const Relax &rx, float *m)
+__device__ __forceinline__ void node_update(const float *f, unsigned type, const Relax &rx, float *m)
 {
-    if (type)
-        zero_unknown<Q>(f, unknown_dirs(type));
     float s[10];
     moment_folds<Q>(f, s);
     if (type)

@@ -32,8 +32,12 @@ __device__ __forceinline__ uint64_t global_ns()
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
     return t;
 }
-// Bounded wait: gives up after `limit_ns` and reports false.
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, unsigned parity, uint64_t limit_ns)
+// Bounded wait: gives up after `limit_ns` and reports false.  With `aborted`
+// (a flag in shared memory) it also gives up, after one round of polls, once
+// the flag is set: a CTA whose earlier wait gave up runs to its end without
+// waiting out the limit again for every copy that is missing.
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, unsigned parity, uint64_t limit_ns,
+                                                  const int *aborted = nullptr)
 {
     if (mbar_try_wait(bar, parity))
         return true;
@@ -43,6 +47,8 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, unsigned parity
             if (mbar_try_wait(bar, parity))
                 return true;
         if (global_ns() - t0 > limit_ns)
+            return false;
+        if (aborted && *reinterpret_cast<const volatile int *>(aborted))
             return false;
     }
 }

@@ -208,14 +208,17 @@ struct ZGroups {
 // S alone on the diagonals).  In the population plane a group's (S, U) pair
 // is one float2 cell and its D one float cell, so a node stores and a
 // neighbour pulls a whole group with two shared-memory accesses.
+// The order of the groups makes every mirror a constant shift of the planes:
+// x-mirrored groups (cx = 1 -> -1) lie 3 groups later, y-mirrored ones
+// (cy = 1 -> -1) the next one, so a ring side and its opposite share code.
 __host__ __device__ constexpr int group_cx(int g)
 {
-    constexpr int t[8] = {1, -1, 0, 0, 1, -1, 1, -1};
+    constexpr int t[8] = {1, 1, 1, -1, -1, -1, 0, 0};
     return t[g];
 }
 __host__ __device__ constexpr int group_cy(int g)
 {
-    constexpr int t[8] = {0, 0, 1, -1, 1, -1, -1, 1};
+    constexpr int t[8] = {1, -1, 0, 1, -1, 0, 1, -1};
     return t[g];
 }
 // direction q of lattice Q with step (cx, cy, cz), or -1
@@ -323,24 +326,66 @@ __device__ __forceinline__ void store_group(float *pb, int cell, const RecPre &r
         pb[C::template d<g>(cell)] = rec_q<Q, qd>(r, m);
 }
 
+// Plane shifts (floats) between the cells of a group and of its mirror along
+// AXIS: SU cells, S-only cells, D cells.
+template <int Q, int AXIS>
+struct MirrorShift {
+    using PG = PopGroups<Q>;
+    // an axis group and a diagonal one, and their mirrors
+    static constexpr int A = AXIS == 0 ? 2 : 6, AM = AXIS == 0 ? 5 : 7, B = 0, BM = AXIS == 0 ? 3 : 1;
+    static constexpr int SU = 2 * (PG::su_plane(AM) - PG::su_plane(A));
+    static constexpr int S = PG::s_plane(BM) - PG::s_plane(B);
+    static constexpr int D = PG::d_plane(AM) - PG::d_plane(A);
+};
+
 // Reconstruct the x-y movers of ring node (rx, ry) that point into the tile
-// (the groups with the given sign of cx or cy) and store them into pop plane pb.
-template <int Q, int TX, int TY, int AXIS, int SIGN, typename ST>
-__device__ __forceinline__ void ring_pops(const ST *sm, float *pb, int rx, int ry)
+// -- those with c_AXIS = +1, or with `neg` their mirrors c_AXIS = -1 -- and
+// store them into pop plane pb.  The mirrored populations are those of the
+// node with the sign of u_AXIS and of the two mixed moments along AXIS
+// flipped (s - m and s + (-m) round alike), so both sides of the ring run
+// the same instructions.  A node outside the domain (live false) has rho = 0
+// and so gives zero populations.
+template <int Q, int TX, int TY, int AXIS, typename ST>
+__device__ __forceinline__ void ring_pops(const ST *sm, float *pb, int rx, int ry, bool neg, bool live)
 {
     using G = TileGeom<TX, TY, ST>;
+    using C = PopCell<Q, TX, TY, ST>;
+    using PG = PopGroups<Q>;
+    using MS = MirrorShift<Q, AXIS>;
     float m[10];
 #pragma unroll
     for (int k = 0; k < 10; k++)
         m[k] = Storage<ST>::load_raw(sm[(k * G::RY + ry + 1) * G::TXP + rx + G::XPAD]);
-    m[0] = rho_of_stored<ST>(m[0]);
+    m[0] = live ? rho_of_stored<ST>(m[0]) : 0.0f;
+    const float sgn = neg ? -1.0f : 1.0f;
+    constexpr int k0 = AXIS == 0 ? 1 : 2, k2 = AXIS == 0 ? 6 : 8;
+    m[k0] *= sgn;
+    m[5] *= sgn;
+    m[k2] *= sgn;
     const RecPre r = rec_pre<Q, Storage<ST>::SCI>(m);
     const int cell = (ry + 1) * G::PX + rx + 1;
-    static_for<0, PopGroups<Q>::NG>([&](auto gc) {
+    float *const su = pb + (neg ? MS::SU * C::PLANE : 0) + 2 * cell;
+    float *const so = pb + (neg ? MS::S * C::PLANE : 0) + cell;
+    float *const dn = pb + (neg ? MS::D * C::PLANE : 0) + cell;
+    static_for<0, PG::NG>([&](auto gc) {
         constexpr int g = decltype(gc)::value;
         constexpr int c = AXIS == 0 ? group_cx(g) : group_cy(g);
-        if constexpr (c == SIGN)
-            store_group<Q, TX, TY, ST, g>(pb, cell, r, m);
+        if constexpr (c == 1) {
+            constexpr int gm = AXIS == 0 ? g + 3 : g + 1;  // the mirrored group
+            constexpr int qs = PG::qS(g), qu = PG::qU(g), qd = PG::qD(g);
+            if constexpr (qu >= 0) {
+                static_assert(2 * (PG::su_plane(gm) - PG::su_plane(g)) == MS::SU, "constant mirror shift");
+                *reinterpret_cast<float2 *>(su + 2 * PG::su_plane(g) * C::PLANE) =
+                    make_float2(rec_q<Q, qs>(r, m), rec_q<Q, qu>(r, m));
+            } else {
+                static_assert(PG::s_plane(gm) - PG::s_plane(g) == MS::S, "constant mirror shift");
+                so[PG::s_plane(g) * C::PLANE] = rec_q<Q, qs>(r, m);
+            }
+            if constexpr (qd >= 0) {
+                static_assert(PG::d_plane(gm) - PG::d_plane(g) == MS::D, "constant mirror shift");
+                dn[PG::d_plane(g) * C::PLANE] = rec_q<Q, qd>(r, m);
+            }
+        }
     });
 }
 
@@ -434,8 +479,11 @@ static __device__ __noinline__ void record_bounds(StepFault *f, unsigned code, i
 // across all the items it processes, so that the stage slot (g % NSTAGE), the
 // phase of its mbarrier ((g / NSTAGE) & 1) and the population plane (g & 1)
 // keep cycling from one item to the next; the mbarriers are initialised once
-// per CTA.  Returns false, uniformly across the CTA, when a TMA wait timed
-// out (the error flag is then set).
+// per CTA.  Returns false, uniformly across the CTA, when a wait timed out
+// (the error flag is then set).  After a TMA wait that timed out the item is
+// marched to its end on whatever the stage holds -- the step is lost and
+// reported, and no plane of a sound step pays for a test of the flag -- but
+// no further copy is issued.
 //
 // CLM selects the relaxation: 0 the plain collision; 1 the learned closure
 // with dtau read per node from p.dtau; 2 the learned closure with the network
@@ -499,6 +547,22 @@ __device__ __forceinline__ bool march_chunk(const CUtensorMap *tmap, const StepP
                      0, &bars[slot], G::PLANE_BYTES);
     }
 
+    bool arrived = true;  // every copy this thread waited for has landed
+    const int lane = lin & 31;
+    // Ring role of this thread's warp (32-wide tiles): 0 bottom row, 1 top
+    // row, 2 both columns, others none.  The roles start at another warp in
+    // neighbouring CTAs, since warp w always issues on scheduler w mod 4 and
+    // the roles would otherwise load the same schedulers in every CTA.
+    const int role = ((lin >> 5) + bx + by + bz) & 7;
+    bool ring_live;  // the ring node this thread reconstructs lies in the mesh (x and y)
+    if constexpr (TX == 32)
+        ring_live = role == 0 ? y0 > 0 && x < p.nx : role == 1 ? y0 + TY < p.ny && x < p.nx
+                    : (lane >= 16 ? x0 + TX < p.nx : x0 > 0) && y0 + (lane & 15) >= 1 && y0 + (lane & 15) <= p.ny;
+    else if (lin < 2 * (TX + 2))
+        ring_live = (lin < TX + 2 ? y0 > 0 : y0 + TY < p.ny) && x0 + lin % (TX + 2) >= 1 && x0 + lin % (TX + 2) <= p.nx;
+    else
+        ring_live = (lin < 2 * (TX + 2) + TY ? x0 > 0 : x0 + TX < p.nx) && y0 + (lin - 2 * (TX + 2)) % TY < p.ny;
+
     // Populations held in registers between planes: the up-movers of the
     // two previous planes (UA for even i, UB for odd i) and the same-plane
     // movers of the previous plane (S1).  The iteration for plane i reads
@@ -527,6 +591,11 @@ __device__ __forceinline__ bool march_chunk(const CUtensorMap *tmap, const StepP
         const uint32_t iu = uint32_t(zu) * plane32 + row32;
         MeanT sm_old[6], km_old = MeanT(0);
         float dtau = 0.0f;
+        // planes outside the mesh (z = -1, z = nz) give zero populations, as
+        // nodes outside it in x and y do: what streams into a boundary node
+        // from outside is zero, and zero terms leave the right folds' values
+        // alone (the reference multiplies those terms by zero)
+        const bool z_in = pz >= 0 && pz < p.nz;
         // this thread updates a node in this iteration (checked build: one in
         // this launch's planes and in the mesh); only such threads touch the
         // node's global fields
@@ -549,9 +618,10 @@ __device__ __forceinline__ bool march_chunk(const CUtensorMap *tmap, const StepP
             }
         }
 
-        if (!mbar_wait_bounded(&bars[stage], parity, p.timeout_ns)) {
+        if (!mbar_wait_bounded(&bars[stage], parity, p.timeout_ns, s_abort)) {
             record_fault(p.fault, ERR_TMA_TIMEOUT, item, mesh, i, g0 + i, stage, parity, &bars[stage]);
             *s_abort = 1;
+            arrived = false;
         }
 
         // own node: reconstruct all directions
@@ -569,7 +639,7 @@ __device__ __forceinline__ bool march_chunk(const CUtensorMap *tmap, const StepP
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 }
             }
-            m[0] = rho_of_stored<ST>(m[0]);
+            m[0] = own && z_in ? rho_of_stored<ST>(m[0]) : 0.0f;
             const RecPre r = rec_pre<Q, Storage<ST>::SCI>(m);
             const int cell = LBM_IDX(my_cell, PCELLS, i);
             static_for<0, PG::NG>([&](auto gc) { store_group<Q, TX, TY, ST, decltype(gc)::value>(pb, cell, r, m); });
@@ -582,11 +652,8 @@ __device__ __forceinline__ bool march_chunk(const CUtensorMap *tmap, const StepP
             // every ring node this thread reconstructs lies on the ring
             int rx = -2, ry = -2;
             if (TX == 32) {
-                const int w = lin >> 5, l = lin & 31;
-                if (w == 0) { rx = l; ry = -1; }
-                else if (w == 1) { rx = l; ry = TY; }
-                else if (w == 2 && l < TY + 2) { rx = -1; ry = l - 1; }
-                else if (w == 3 && l < TY + 2) { rx = TX; ry = l - 1; }
+                if (role < 2) { rx = lane; ry = role ? TY : -1; }
+                else if (role == 2 && (lane & 15) < TY + 2) { rx = lane >= 16 ? TX : -1; ry = (lane & 15) - 1; }
             } else if (lin < G::RING) {
                 int r = lin;
                 if (r < TX + 2) { rx = r - 1; ry = -1; }
@@ -600,48 +667,44 @@ __device__ __forceinline__ bool march_chunk(const CUtensorMap *tmap, const StepP
         }
 #endif
         // ring nodes: only the directions that enter the tile.  With 32-wide
-        // tiles each side goes to one warp (the bottom and top rows, x = 0..31,
-        // to warps 0 and 1; the left and right columns, corners included, to
-        // warps 2 and 3), so no warp runs two sides one after the other.
+        // tiles the bottom and top rows (x = 0..31) take one warp each and
+        // the left and right columns (corners included) share a third, so no
+        // warp runs two sides one after the other.
         if constexpr (TX == 32) {
-            const int w = lin >> 5, l = lin & 31;
-            if (w == 0) {
-                ring_pops<Q, TX, TY, 1, +1, ST>(sm, pb, l, -1);
-            } else if (w == 1) {
-                ring_pops<Q, TX, TY, 1, -1, ST>(sm, pb, l, TY);
-            } else if (w == 2) {
-                if (l < TY + 2)
-                    ring_pops<Q, TX, TY, 0, +1, ST>(sm, pb, -1, l - 1);
-            } else if (w == 3) {
-                if (l < TY + 2)
-                    ring_pops<Q, TX, TY, 0, -1, ST>(sm, pb, TX, l - 1);
+            static_assert(TY + 2 <= 16, "both columns fit one warp");
+            if (role < 2) {
+                const int ry = role ? TY : -1;
+                ring_pops<Q, TX, TY, 1, ST>(sm, pb, lane, ry, role != 0, z_in && ring_live);
+            } else if (role == 2 && (lane & 15) < TY + 2) {
+                const int rx = lane >= 16 ? TX : -1;
+                ring_pops<Q, TX, TY, 0, ST>(sm, pb, rx, (lane & 15) - 1, lane >= 16, z_in && ring_live);
             }
         } else if (lin < G::RING) {
             int r = lin;
-            if (r < TX + 2) {
-                ring_pops<Q, TX, TY, 1, +1, ST>(sm, pb, r - 1, -1);
-            } else if ((r -= TX + 2) < TX + 2) {
-                ring_pops<Q, TX, TY, 1, -1, ST>(sm, pb, r - 1, TY);
-            } else if ((r -= TX + 2) < TY) {
-                ring_pops<Q, TX, TY, 0, +1, ST>(sm, pb, -1, r);
+            if (r < 2 * (TX + 2)) {
+                const bool top = r >= TX + 2;
+                const int rx = r - (top ? TX + 2 : 0) - 1, ry = top ? TY : -1;
+                ring_pops<Q, TX, TY, 1, ST>(sm, pb, rx, ry, top, z_in && ring_live);
             } else {
-                r -= TY;
-                ring_pops<Q, TX, TY, 0, -1, ST>(sm, pb, TX, r);
+                r -= 2 * (TX + 2);
+                const bool right = r >= TY;
+                const int rx = right ? TX : -1, ry = r - (right ? TY : 0);
+                ring_pops<Q, TX, TY, 0, ST>(sm, pb, rx, ry, right, z_in && ring_live);
             }
         }
         if constexpr (CLM == 2)
             tc_fence_before();
         cta_sync();
-        if (*s_abort)
-            return false;
         if constexpr (CLM == 2) {
+            if (*s_abort)
+                return false;
             if (net_plane)
                 fused_issue_layer1(*mlp);
         }
 
         // the stage is consumed: refill it with plane i + NSTAGE
         (void)LBM_CHK(!(lin == 0 && i + NSTAGE < nplanes) || (pz + NSTAGE <= p.nz && pz + NSTAGE <= z1), CHK_TMA_PLANE, i);
-        tma_issue_if(lin == 0 && i + NSTAGE < nplanes, sm, tmap, x0 - G::XPAD, y0 - 1, pz + NSTAGE, 0, &bars[stage],
+        tma_issue_if(lin == 0 && arrived && i + NSTAGE < nplanes, sm, tmap, x0 - G::XPAD, y0 - 1, pz + NSTAGE, 0, &bars[stage],
                      G::PLANE_BYTES);
 
         // pull the down-movers (cz = -1) that land on plane pz-1
@@ -799,7 +862,7 @@ __device__ __forceinline__ bool march_chunk(const CUtensorMap *tmap, const StepP
                 return false;
         }
     }
-    return true;
+    return *s_abort == 0;
 }
 
 // CTA sums of the monitor, then one FP64 atomic per quantity.
