@@ -549,11 +549,12 @@ __device__ __forceinline__ bool march_chunk(const CUtensorMap *tmap, const StepP
 
     bool arrived = true;  // every copy this thread waited for has landed
     const int lane = lin & 31;
+    const int warp = __shfl_sync(0xffffffffu, lin >> 5, 0);  // the same for the whole warp, known as such
     // Ring role of this thread's warp (32-wide tiles): 0 bottom row, 1 top
     // row, 2 both columns, others none.  The roles start at another warp in
     // neighbouring CTAs, since warp w always issues on scheduler w mod 4 and
     // the roles would otherwise load the same schedulers in every CTA.
-    const int role = ((lin >> 5) + bx + by + bz) & 7;
+    const int role = (warp + bx + by + bz) & 7;
     bool ring_live;  // the ring node this thread reconstructs lies in the mesh (x and y)
     if constexpr (TX == 32)
         ring_live = role == 0 ? y0 > 0 && x < p.nx : role == 1 ? y0 + TY < p.ny && x < p.nx
@@ -702,10 +703,13 @@ __device__ __forceinline__ bool march_chunk(const CUtensorMap *tmap, const StepP
                 fused_issue_layer1(*mlp);
         }
 
-        // the stage is consumed: refill it with plane i + NSTAGE
+        // the stage is consumed: refill it with plane i + NSTAGE (the branch
+        // is uniform per warp, so it splits none; predicating the issue in
+        // every warp instead cost 15 of 581 instructions per D3Q27 node)
         (void)LBM_CHK(!(lin == 0 && i + NSTAGE < nplanes) || (pz + NSTAGE <= p.nz && pz + NSTAGE <= z1), CHK_TMA_PLANE, i);
-        tma_issue_if(lin == 0 && arrived && i + NSTAGE < nplanes, sm, tmap, x0 - G::XPAD, y0 - 1, pz + NSTAGE, 0, &bars[stage],
-                     G::PLANE_BYTES);
+        if (warp == 0)
+            tma_issue_if(lane == 0 && arrived && i + NSTAGE < nplanes, sm, tmap, x0 - G::XPAD, y0 - 1, pz + NSTAGE, 0,
+                         &bars[stage], G::PLANE_BYTES);
 
         // pull the down-movers (cz = -1) that land on plane pz-1
         static_for<0, PG::NG>([&](auto gc) {
