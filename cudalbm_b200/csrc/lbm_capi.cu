@@ -512,7 +512,10 @@ lbm_status launch_step(lbm_handle *h, bool monitored = false)
     p.nx = int(h->cfg.nx);
     p.ny = int(h->cfg.ny);
     p.nz = int(h->cfg.nz);
-    p.zc = h->zc;
+    const lbm::ZChunks zch = lbm::handle_chunks(h);
+    p.zc = zch.zc;
+    p.nbig = zch.nbig;
+    p.zc2 = zch.zc2;
     p.z_lo = 0;
     p.z_hi = p.nz;
     p.rx = lbm::Relax{h->omega, h->t_omega, h->omega_d2, h->tau, h->cfg.u_inf};
@@ -537,7 +540,7 @@ lbm_status launch_step(lbm_handle *h, bool monitored = false)
     const dim3 block(h->launcher.tx, h->launcher.ty);
     const dim3 grid(unsigned((h->cfg.nx + h->launcher.tx - 1) / h->launcher.tx),
                     unsigned((h->cfg.ny + h->launcher.ty - 1) / h->launcher.ty),
-                    unsigned((h->cfg.nz + h->zc - 1) / h->zc));
+                    unsigned(zch.count));
     void *args[] = {&h->tmap[h->cur], &p};
     LBM_CUDA(cudaLaunchKernel(monitored ? h->launcher.fn_mon : h->launcher.fn, grid, block, args, h->launcher.smem,
                               h->stream));
@@ -559,7 +562,8 @@ lbm_status launch_slab(lbm_handle *h, int in, int64_t t, int z_lo, int z_hi, int
     p.nx = int(h->cfg.nx);
     p.ny = int(h->cfg.ny);
     p.nz = int(h->cfg.nz);
-    p.zc = zc;
+    p.zc = p.zc2 = zc;
+    p.nbig = 0;
     p.z_lo = z_lo;
     p.z_hi = z_hi;
     p.rx = lbm::Relax{h->omega, h->t_omega, h->omega_d2, h->tau, h->cfg.u_inf};

@@ -560,7 +560,10 @@ lbm_status closure_step(lbm_handle *h)
         p.nx = int(h->cfg.nx);
         p.ny = int(h->cfg.ny);
         p.nz = int(h->cfg.nz);
-        p.zc = h->zc;
+        const ZChunks zch = handle_chunks(h);
+        p.zc = zch.zc;
+        p.nbig = zch.nbig;
+        p.zc2 = zch.zc2;
         p.z_lo = 0;
         p.z_hi = p.nz;
         p.rx = Relax{h->omega, h->t_omega, h->omega_d2, h->tau, h->cfg.u_inf};
@@ -570,7 +573,7 @@ lbm_status closure_step(lbm_handle *h)
         const dim3 block(h->launcher.tx, h->launcher.ty);
         const dim3 grid(unsigned((h->cfg.nx + h->launcher.tx - 1) / h->launcher.tx),
                         unsigned((h->cfg.ny + h->launcher.ty - 1) / h->launcher.ty),
-                        unsigned((h->cfg.nz + h->zc - 1) / h->zc));
+                        unsigned(zch.count));
         void *args[] = {&h->tmap[h->cur], &p, &net};
         LBM_CUDA_RETURN(cudaLaunchKernel(ffn, grid, block, args, fsmem, h->stream));
         h->closure_steps++;
@@ -599,7 +602,10 @@ lbm_status closure_step(lbm_handle *h)
     p.nx = int(h->cfg.nx);
     p.ny = int(h->cfg.ny);
     p.nz = int(h->cfg.nz);
-    p.zc = h->zc;
+    const ZChunks zch = handle_chunks(h);
+    p.zc = zch.zc;
+    p.nbig = zch.nbig;
+    p.zc2 = zch.zc2;
     p.z_lo = 0;
     p.z_hi = p.nz;
     p.rx = Relax{h->omega, h->t_omega, h->omega_d2, h->tau, h->cfg.u_inf};
@@ -609,7 +615,7 @@ lbm_status closure_step(lbm_handle *h)
     const dim3 block(h->launcher.tx, h->launcher.ty);
     const dim3 grid(unsigned((h->cfg.nx + h->launcher.tx - 1) / h->launcher.tx),
                     unsigned((h->cfg.ny + h->launcher.ty - 1) / h->launcher.ty),
-                    unsigned((h->cfg.nz + h->zc - 1) / h->zc));
+                    unsigned(zch.count));
     void *args[] = {&h->tmap[h->cur], &p};
     LBM_CUDA_RETURN(cudaLaunchKernel(fn, grid, block, args, smem, h->stream));
     h->cur = nxt;

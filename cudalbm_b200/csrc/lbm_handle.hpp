@@ -68,6 +68,13 @@ struct lbm_handle {
 
 namespace lbm {
 
+// The z-chunks of a whole-mesh step of this handle.
+inline ZChunks handle_chunks(const lbm_handle *h)
+{
+    const int tx = h->launcher.tx, ty = h->launcher.ty;
+    return z_chunks(h->cfg.nz, h->zc, ((h->cfg.nx + tx - 1) / tx) * ((h->cfg.ny + ty - 1) / ty), tx * ty / 32);
+}
+
 // Sets the message returned by lbm_last_error() and returns s.
 lbm_status record_error(lbm_status s, const std::string &msg);
 

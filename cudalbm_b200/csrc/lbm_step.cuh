@@ -147,8 +147,10 @@ struct StepParams {
     ST *out;           // [10][N] moments after the step
     MonitorSlot *mon;  // per-step sums (monitored kernels only)
     int nx, ny, nz;
-    int zc;            // z-planes per CTA
-    int z_lo, z_hi;    // planes this launch updates: CTA bz takes [z_lo + bz zc, min(z_lo + (bz+1) zc, z_hi))
+    // Planes this launch updates and how CTAs share them: the first nbig
+    // chunks of [z_lo, z_hi) have zc planes, the others zc2 (see z_chunks).
+    int zc, nbig, zc2;
+    int z_lo, z_hi;
     Relax rx;
     FOPtrs<MeanT> fo;
     StepFault *fault;
@@ -170,6 +172,28 @@ static_assert(offsetof(StepParamsF32, fault) == offsetof(StepParamsF64Means, fau
                   offsetof(StepParamsF32, timeout_ns) == offsetof(StepParamsF64Means, timeout_ns) &&
                   offsetof(StepParamsF32, dtau) == offsetof(StepParamsF64Means, dtau),
               "fields after the function-object block at the same offsets for both mean precisions");
+
+// How `nz` planes are cut into z-chunks for tiles of `warps` warps, `tiles` of
+// them per plane.  A chunk of zc planes reconstructs zc + 2, so long chunks
+// save work, but the grid's last CTAs then run alone for a whole long chunk.
+// With at least two waves of work on the GPU (24 warps per SM are resident)
+// the end of z, 3/4 to 7/4 of a chunk, is therefore cut into quarter chunks;
+// CTAs start in the order of their chunk, so these fill the end of the grid.
+// 256^3, us per step, best uniform chunk (19) / 32 + quarters: D3Q27 334.1 /
+// 325.5, D3Q19 250.4 / 246.8, D3Q19 FP16 245.7 / 239.8; with 26 + quarters
+// D3Q27 with S/SMean/k/kMean 486.7 / 484.1.
+struct ZChunks {
+    int zc, nbig, zc2, count;
+};
+inline ZChunks z_chunks(int64_t nz, int zc, int64_t tiles, int warps)
+{
+    const int uniform = int((nz + zc - 1) / zc);
+    constexpr int64_t kSms = 148, kResidentWarps = 24;
+    if (zc < 16 || tiles * uniform * warps < 2 * kSms * kResidentWarps || nz < 2 * zc)
+        return {zc, uniform, zc, uniform};
+    const int nbig = int((nz - (3 * zc + 3) / 4) / zc), zc2 = (zc + 3) / 4;
+    return {zc, nbig, zc2, nbig + int((nz - int64_t(nbig) * zc + zc2 - 1) / zc2)};
+}
 
 template <int TX, int TY, typename ST = float>
 struct TileGeom {
@@ -508,8 +532,8 @@ __device__ __forceinline__ bool march_chunk(const CUtensorMap *tmap, const StepP
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int lin = ty * TX + tx;
     const int x0 = bx * TX, y0 = by * TY;
-    const int z0 = p.z_lo + bz * p.zc;
-    const int z1 = min(z0 + p.zc, p.z_hi);
+    const int z0 = p.z_lo + bz * p.zc - max(bz - p.nbig, 0) * (p.zc - p.zc2);
+    const int z1 = min(z0 + (bz < p.nbig ? p.zc : p.zc2), p.z_hi);
     const int nplanes = z1 - z0 + 2;  // planes z0-1 .. z1
     const int x = x0 + tx, y = y0 + ty;
     const bool own = (x < p.nx) && (y < p.ny);
@@ -1146,7 +1170,8 @@ __global__ void __launch_bounds__(TX *TY, MINB) batch_kernel(const BatchParams b
         p.nx = bm.nx;
         p.ny = bm.ny;
         p.nz = bm.nz;
-        p.zc = bm.zc;
+        p.zc = p.zc2 = bm.zc;
+        p.nbig = 0;
         p.z_lo = 0;
         p.z_hi = bm.nz;
         p.rx = bm.rx;

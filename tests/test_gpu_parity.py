@@ -68,6 +68,17 @@ def test_tiling_and_chunking_do_not_change_results(q, tile, z_chunk):
         assert bits_equal(out[k], base[k]), k
 
 
+@pytest.mark.parametrize("q,nx,fo", [(19, 256, ()), (27, 264, ("S", "kMean"))])
+@pytest.mark.parametrize("z_chunk", [16, 23, 32])
+def test_tapered_chunks_equal_uniform_ones(q, nx, fo, z_chunk):
+    """A grid of two waves or more ends in quarter chunks (z_chunks); the
+    same bits as uniform short chunks, the last tile partly outside the mesh."""
+    base = run_cavity(q, nx, 256, 72, 400.0, 0.05, 5, fo=fo, tile=(32, 8, 2), z_chunk=8)
+    out = run_cavity(q, nx, 256, 72, 400.0, 0.05, 5, fo=fo, tile=(32, 8, 2), z_chunk=z_chunk)
+    for k in base:
+        assert bits_equal(out[k], base[k]), k
+
+
 @pytest.mark.parametrize("q", [19, 27])
 def test_against_fp64_oracle(q):
     n = (24, 16, 32)
