@@ -133,8 +133,8 @@ lbm_status launch(lbm_batch *b, int flip)
 {
     lbm::BatchParams p = params_of(b);
     void *args[] = {&p, &flip};
-    LBM_CUDA_RETURN(cudaLaunchKernel(b->launcher.fn, dim3(b->grid), dim3(b->launcher.tx, b->launcher.ty), args,
-                                     b->launcher.smem, b->stream));
+    LBM_CUDA_RETURN(lbm::launch_overlapped(b->launcher.fn, dim3(b->grid), dim3(b->launcher.tx, b->launcher.ty), args,
+                                           b->launcher.smem, b->stream));
     b->launches += 1;
     return LBM_OK;
 }

@@ -542,8 +542,8 @@ lbm_status launch_step(lbm_handle *h, bool monitored = false)
                     unsigned((h->cfg.ny + h->launcher.ty - 1) / h->launcher.ty),
                     unsigned(zch.count));
     void *args[] = {&h->tmap[h->cur], &p};
-    LBM_CUDA(cudaLaunchKernel(monitored ? h->launcher.fn_mon : h->launcher.fn, grid, block, args, h->launcher.smem,
-                              h->stream));
+    LBM_CUDA(lbm::launch_overlapped(monitored ? h->launcher.fn_mon : h->launcher.fn, grid, block, args,
+                                    h->launcher.smem, h->stream));
     h->cur = nxt;
     h->t += 1;
     h->launches += 1;
@@ -602,6 +602,21 @@ lbm_status record_error(lbm_status s, const std::string &msg)
 }
 
 EncodeTiledFn encode_tiled() { return get_encode(); }
+
+cudaError_t launch_overlapped(const void *fn, dim3 grid, dim3 block, void **args, size_t smem, cudaStream_t stream)
+{
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelExC(&cfg, fn, args);
+}
 
 lbm_status check_fault(const StepFault &f, const char *who)
 {

@@ -575,7 +575,7 @@ lbm_status closure_step(lbm_handle *h)
                         unsigned((h->cfg.ny + h->launcher.ty - 1) / h->launcher.ty),
                         unsigned(zch.count));
         void *args[] = {&h->tmap[h->cur], &p, &net};
-        LBM_CUDA_RETURN(cudaLaunchKernel(ffn, grid, block, args, fsmem, h->stream));
+        LBM_CUDA_RETURN(launch_overlapped(ffn, grid, block, args, fsmem, h->stream));
         h->closure_steps++;
         h->dtau_current = false;
         h->last_input_kept = true;
@@ -617,7 +617,7 @@ lbm_status closure_step(lbm_handle *h)
                     unsigned((h->cfg.ny + h->launcher.ty - 1) / h->launcher.ty),
                     unsigned(zch.count));
     void *args[] = {&h->tmap[h->cur], &p};
-    LBM_CUDA_RETURN(cudaLaunchKernel(fn, grid, block, args, smem, h->stream));
+    LBM_CUDA_RETURN(launch_overlapped(fn, grid, block, args, smem, h->stream));
     h->cur = nxt;
     h->t += 1;
     h->launches += 1;

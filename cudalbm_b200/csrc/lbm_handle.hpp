@@ -84,6 +84,10 @@ using EncodeTiledFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_
                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 EncodeTiledFn encode_tiled();
 
+// Launch of a step kernel that may start before the kernel in front of it in
+// the stream has ended (it waits by itself, see wait_previous_grid).
+cudaError_t launch_overlapped(const void *fn, dim3 grid, dim3 block, void **args, size_t smem, cudaStream_t stream);
+
 // Frees a handle regardless of batch ownership (used by lbm_batch_destroy).
 void destroy_handle(lbm_handle *h);
 

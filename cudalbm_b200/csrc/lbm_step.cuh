@@ -957,9 +957,11 @@ __global__ void __launch_bounds__(TX *TY, MINB)
     init_barriers<NSTAGE>(sh.bars, lin == 0);
     s_abort = 0;
     cta_sync();
+    wait_previous_grid();
     MonAcc acc;
     march_chunk<Q, TX, TY, NSTAGE, FO, MeanT, MON, NPB, ST>(&tmap_in, p, blockIdx.x, blockIdx.y, blockIdx.z, 0u, sh,
                                                             &s_abort, acc);
+    let_next_grid_start();
     if constexpr (MON)
         monitor_flush<TX * TY>(acc, p.mon, lin);
     if (s_abort && lin == 0)
@@ -979,9 +981,11 @@ __global__ void __launch_bounds__(TX *TY, MINB)
     init_barriers<NSTAGE>(sh.bars, lin == 0);
     s_abort = 0;
     cta_sync();
+    wait_previous_grid();
     MonAcc acc;
     march_chunk<Q, TX, TY, NSTAGE, false, float, false, NPB, float, 1>(&tmap_in, p, blockIdx.x, blockIdx.y,
                                                                        blockIdx.z, 0u, sh, &s_abort, acc);
+    let_next_grid_start();
     if (s_abort && lin == 0)
         drain_after_abort<NSTAGE>(sh.bars);
 }
@@ -1044,6 +1048,7 @@ __global__ void __launch_bounds__(TX *TY, MINB)
     cta_sync();
     tc_fence_after();
     const uint32_t tbase = *tslot;
+    wait_previous_grid();
     FusedMlp f;
     f.w1 = reinterpret_cast<__half *>(ms + MS::W1);
     f.w2 = reinterpret_cast<__half *>(ms + MS::W2);
@@ -1065,6 +1070,7 @@ __global__ void __launch_bounds__(TX *TY, MINB)
     march_chunk<Q, TX, TY, NSTAGE, false, float, false, NPB, float, 2>(&tmap_in, p, blockIdx.x, blockIdx.y,
                                                                        blockIdx.z, 0u, sh, &s_abort, acc, -1, -1,
                                                                        &f, &net);
+    let_next_grid_start();
     if (s_abort) {
         if (lin == 0)
             drain_after_abort<NSTAGE>(sh.bars);
@@ -1132,6 +1138,7 @@ __global__ void __launch_bounds__(TX *TY, MINB) batch_kernel(const BatchParams b
     const int lin = threadIdx.y * TX + threadIdx.x;
     init_barriers<NSTAGE>(sh.bars, lin == 0);
     s_abort = 0;
+    wait_previous_grid();
     MonAcc acc;
     unsigned g = 0;  // planes received so far by this CTA
     for (int round = 0;; round++) {
@@ -1187,6 +1194,7 @@ __global__ void __launch_bounds__(TX *TY, MINB) batch_kernel(const BatchParams b
             break;
         g += unsigned(min(p.zc, p.nz - bz * p.zc) + 2);
     }
+    let_next_grid_start();
     if (lin == 0) {
         if (s_abort)
             drain_after_abort<NSTAGE>(sh.bars);
