@@ -250,19 +250,48 @@ bool pick_launcher(int Q, int tx, int ty, int stages, int npb, int storage, unsi
                    : lbm::pick_q27_f32(tx, ty, stages, npb, fo, mean_bits, out);
 }
 
-// Default tiling for a mesh: widest tile whose width divides nx, z-chunks
-// sized so that the grid holds several waves of CTAs on 148 SMs.
-void default_tiling(int Q, int64_t nx, int64_t ny, int64_t nz, int &tx, int &ty, int &zc, int &stages)
+// Default kernel shape of a mesh: the tile width and z-chunk with the least
+// predicted time per step.  A plane of the march costs every SM
+// max(floor, base + per_cta * n) us with n CTAs on it (D3Q19, FP32; D3Q27 takes
+// 1.25 times as long in every term, so the choice is the same): the floor is
+// the chain of one plane -- copy, reconstruction, barrier, update -- that a
+// lone CTA waits out, per_cta the issue slots of a tile.  A grid with a
+// tapered end (z_chunks) is charged for the planes its CTAs visit and half a
+// chunk of draining.  Tiles with more than half of their lanes outside the
+// mesh are left out.  Over 38 meshes from 32x16x24 to 192^3 the choice is
+// within 15% of the fastest (tile, z-chunk), 3% on average.  D3Q19, us per
+// step, the former rule (widest tile that divides nx, chunks of 9 or more) ->
+// this one: 32x16x24 16.4 -> 4.1, 8x64x64 24.1 -> 5.2, 64^3 20.3 -> 9.5,
+// 88x96x104 30.0 -> 24.9, 296x264x248 690 -> 317.
+void default_tiling(int64_t nx, int64_t ny, int64_t nz, int only_tx, bool narrow, int &tx, int &zc)
 {
-    (void)Q;
-    tx = (nx % 32 == 0) ? 32 : (nx % 16 == 0 ? 16 : 8);
-    ty = 8;
-    stages = 2;
-    const int64_t tiles = ((nx + tx - 1) / tx) * ((ny + ty - 1) / ty);
-    int64_t c = nz;
-    while (c > 16 && tiles * ((nz + c - 1) / c) < 8 * 148)
-        c = (c + 1) / 2;
-    zc = int(c);
+    struct Tile {
+        int tx;
+        double floor, base, per_cta;
+    };
+    constexpr Tile kTiles[] = {{32, 1.1, 0.33, 0.55}, {16, 1.1, 0.6, 0.29}, {8, 1.1, 0.6, 0.21}};
+    constexpr double kSms = 148.0;
+    double best = 1e300;
+    for (const Tile &t : kTiles) {
+        if (only_tx ? t.tx != only_tx : (t.tx == 8 && !narrow) || (t.tx > 8 && nx <= t.tx / 2 && (narrow || t.tx > 16)))
+            continue;
+        const int64_t tiles = ((nx + t.tx - 1) / t.tx) * ((ny + 7) / 8);
+        for (int c : {1, 2, 3, 4, 6, 8, 11, 16, 26}) {
+            if (c > nz)
+                continue;
+            const lbm::ZChunks z = lbm::z_chunks(nz, c, tiles, t.tx * 8 / 32);
+            double us;
+            if (z.zc2 != z.zc)
+                us = t.per_cta * double(tiles) * double(nz + 2 * z.count) / kSms + 0.5 * t.base * (c + 2);
+            else
+                us = (c + 2) * std::max(t.floor, t.base + t.per_cta * std::ceil(double(tiles) * z.count / kSms));
+            if (us < best) {
+                best = us;
+                tx = t.tx;
+                zc = c;
+            }
+        }
+    }
 }
 
 using lbm::EncodeTiledFn;
@@ -760,16 +789,25 @@ lbm_status lbm_create(const lbm_config *cfg, lbm_handle **out)
     h->t_omega = 1.0f - h->omega;
     h->omega_d2 = h->omega * 0.5f;
 
-    int tx, ty, zc, st;
-    default_tiling(h->Q, c.nx, c.ny, c.nz, tx, ty, zc, st);
+    // A configuration that names a part of the kernel's shape other than its
+    // z-chunk goes with the widest tile that divides nx (pop_buffers and
+    // stages exist for some tiles only, so the tile must not depend on more).
+    int tx = c.nx % 32 == 0 ? 32 : (c.nx % 16 == 0 ? 16 : 8), ty = 8, zc = 0, st = 2;
+    const bool named = c.tile_x || c.tile_y || c.stages || c.pop_buffers;
     if (c.tile_x) tx = c.tile_x;
     if (c.tile_y) ty = c.tile_y;
-    if (c.z_chunk) zc = c.z_chunk;
     if (c.stages) st = c.stages;
-    const unsigned fo = c.function_objects;
-    const int npb = c.pop_buffers ? c.pop_buffers : 1;
     if (h->storage && tx == 8)
         tx = 16;
+    default_tiling(c.nx, c.ny, c.nz, named ? tx : 0, h->storage == 0, tx, zc);
+    if (c.z_chunk) zc = c.z_chunk;
+    const unsigned fo = c.function_objects;
+    // D3Q19 without function objects fits four CTAs per SM at 64 registers;
+    // grids with more than three per SM gain (256^3 258.6 -> 248.3 us per
+    // step, FP16 262 -> 243), smaller ones have no use for the fourth
+    const int64_t ctas = ((c.nx + 31) / 32) * ((c.ny + 7) / 8) * ((c.nz + std::max(zc, 1) - 1) / std::max(zc, 1));
+    const bool four = !named && h->Q == 19 && !fo && tx == 32 && ctas > 3 * 148;
+    const int npb = c.pop_buffers ? c.pop_buffers : (four ? 4 : 1);
     if (!pick_launcher(h->Q, tx, ty, st, npb, h->storage, fo, c.mean_bits, h->launcher)) {
         delete h;
         return fail(LBM_ERR_ARG, "unsupported tile configuration");
@@ -1706,11 +1744,12 @@ lbm_status lbm_autotune(lbm_handle *h, int32_t trial_steps, lbm_tuning *out)
         // (such a chunk re-reads two planes for every 2-4 it updates)
         const int64_t tiles = ((h->cfg.nx + v.tx - 1) / v.tx) * ((h->cfg.ny + v.ty - 1) / v.ty);
         const bool small = tiles * ((h->cfg.nz + 7) / 8) < 4 * 148 * 3;
-        // Candidates: powers of two, and chunk lengths whose grid is close to
-        // a whole number of waves of resident CTAs (k waves for k = 1..12):
-        // the last wave of a grid 9.2 waves long runs the GPU at a fifth of
-        // its CTA slots.  Chunks need not divide nz (the last is shorter).
-        std::vector<int> zcs = {2, 4, 8, 16, 32, 64};
+        // Candidates: a ladder of lengths, and, where the grid's end is not
+        // tapered (z_chunks), those whose grid is close to a whole number of
+        // waves of resident CTAs (k waves for k = 1..12): the last wave of a
+        // grid 9.2 waves long runs the GPU at a fifth of its CTA slots.
+        // Chunks need not divide nz (the last is shorter).
+        std::vector<int> zcs = {1, 2, 3, 4, 6, 8, 11, 16, 20, 26, 32, 37, 43, 52, 64};
         {
             Launcher l;
             int per_sm = 0;
@@ -1723,7 +1762,8 @@ lbm_status lbm_autotune(lbm_handle *h, int32_t trial_steps, lbm_tuning *out)
                 for (int64_t k = 1; k <= 12; k++) {
                     const int64_t chunks = std::max<int64_t>(1, (k * resident + tiles / 2) / tiles);
                     const int zc = int((h->cfg.nz + chunks - 1) / chunks);
-                    if (std::find(zcs.begin(), zcs.end(), zc) == zcs.end())
+                    const lbm::ZChunks z = lbm::z_chunks(h->cfg.nz, zc, tiles, v.tx * v.ty / 32);
+                    if (z.zc2 == z.zc && std::find(zcs.begin(), zcs.end(), zc) == zcs.end())
                         zcs.push_back(zc);
                 }
             }

@@ -1126,8 +1126,7 @@ lbm_status lbm_closure_set(lbm_handle *h, const lbm_mlp *net)
     size_t smem;
     if (!pick_closure(h->Q, h->launcher.tx, h->launcher.ty, h->launcher.stages, h->launcher.pop_buffers, fn, smem)) {
         // move to the closure's kernel shape (same results, other tiling)
-        const int tx = h->cfg.nx % 32 == 0 ? 32 : (h->cfg.nx % 16 == 0 ? 16 : 8);
-        lbm_status s = lbm::retile(h, tx, 8, 2, 1, h->zc);
+        lbm_status s = lbm::retile(h, h->launcher.tx, 8, 2, 1, h->zc);
         if (s != LBM_OK)
             return s;
         pick_closure(h->Q, h->launcher.tx, h->launcher.ty, h->launcher.stages, h->launcher.pop_buffers, fn, smem);

@@ -80,6 +80,17 @@ def test_tapered_chunks_equal_uniform_ones(q, nx, fo, z_chunk):
 
 
 @pytest.mark.parametrize("q", [19, 27])
+@pytest.mark.parametrize("shape,storage", [((8, 8, 8), "f32"), ((16, 24, 40), "f32"), ((40, 16, 24), "f32"),
+                                           ((8, 64, 64), "f32"), ((72, 72, 72), "f32"), ((264, 136, 80), "f32"),
+                                           ((8, 24, 16), "f16"), ((40, 64, 24), "bf16")])
+def test_default_shape_equals_a_named_one(q, shape, storage):
+    """The kernel shape chosen for a mesh gives the bits of 16-wide tiles."""
+    base = run_cavity(q, *shape, 400.0, 0.05, 21, storage=storage, tile=(16, 8, 2), z_chunk=8, pop_buffers=1)
+    out = run_cavity(q, *shape, 400.0, 0.05, 21, storage=storage)
+    assert bits_equal(out["moments"], base["moments"])
+
+
+@pytest.mark.parametrize("q", [19, 27])
 def test_against_fp64_oracle(q):
     n = (24, 16, 32)
     out = run_cavity(q, *n, 250.0, 0.05, 60, fo=("S", "SMean", "k", "kMean", "momentsMean"))
