@@ -477,17 +477,16 @@ __device__ __forceinline__ void scale_collide(float *m, const Relax &rx)
     m[8] = rx.t_omega * m[8] + om * (m[2]) * (m[3]);
 }
 
-// Full node update from the streamed populations f[Q] (in direction order;
-// those that come from outside the mesh are zero, so that the folds of a
-// boundary node are the sums over its known populations: the reference sums
-// incomingSwitch * f_q with incomingSwitch in {0, 1}, velocitySet.cuh:204-220,
-// and a zero term leaves a right fold's value unchanged).
+// Node update from the folds of the streamed populations (moment_folds of
+// f[Q] in direction order, those that come from outside the mesh zero, so that
+// the folds of a boundary node are the sums over its known populations: the
+// reference sums incomingSwitch * f_q with incomingSwitch in {0, 1},
+// velocitySet.cuh:204-220, and a zero term leaves a right fold's value
+// unchanged).
 // Returns the stored (post-collision) moments with rho still including rho0.
 template <int Q, int SCI = 1>
-__device__ __forceinline__ void node_update(const float *f, unsigned type, const Relax &rx, float *m)
+__device__ __forceinline__ void node_update(const float *s, unsigned type, const Relax &rx, float *m)
 {
-    float s[10];
-    moment_folds<Q>(f, s);
     if (type)
         boundary_moments<Q>(s, type, rx, m);
     else

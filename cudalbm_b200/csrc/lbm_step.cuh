@@ -514,8 +514,9 @@ static __device__ __noinline__ void record_bounds(StepFault *f, unsigned code, i
 // evaluated in this kernel (mlp: the thread's group state, net: the network;
 // see FusedMlp), the same dtau as mode 1 after mlp_infer_kernel, bit for bit.
 // FO selects the function objects: 0 none; 1 those whose pointers in p.fo
-// are set (checked per field at run time); 2 exactly S, SMean, k and kMean
-// (the checks resolved at compile time, which measured 3% faster).
+// are set (checked per field at run time), momentsMean not; 2 exactly S, SMean,
+// k and kMean (the checks resolved at compile time, which measured 3% faster);
+// 3 momentsMean and those whose pointers are set.
 template <int Q, int TX, int TY, int NSTAGE, int FO, typename MeanT, bool MON, int NPB, typename ST, int CLM = 0>
 __device__ __forceinline__ bool march_chunk(const CUtensorMap *tmap, const StepParams<MeanT, ST> &p, int bx, int by,
                                             int bz, unsigned g0, const CtaSmem<ST> &sh, int *s_abort, MonAcc &acc,
@@ -546,7 +547,7 @@ __device__ __forceinline__ bool march_chunk(const CUtensorMap *tmap, const StepP
     using PG = PopGroups<Q>;
     using C = PopCell<Q, TX, TY, ST>;
     static_assert(PG::d_plane(PG::NG) == XY<Q>::N, "population-plane groups cover the x-y movers");
-    constexpr bool FO4 = FO == 2;  // S, SMean, k, kMean present, momentsMean absent
+    constexpr bool FO4 = FO == 2;  // S, SMean, k, kMean present
     const int my_cell = (ty + 1) * G::PX + tx + 1;
     constexpr int PCELLS = G::PX * G::PY;  // cells of one population-plane group
 #ifdef LBM_CHECKED
@@ -558,7 +559,7 @@ __device__ __forceinline__ bool march_chunk(const CUtensorMap *tmap, const StepP
         (void)LBM_CHK(z0 >= 0 && z0 < z1 && z1 <= p.nz && z0 >= p.z_lo && z1 <= p.z_hi, CHK_TMA_PLANE, 0);
         (void)LBM_CHK(ty + 1 < G::RY && tx + G::XPAD < G::TXP, CHK_STAGE, 0);
         (void)LBM_CHK(p.out != nullptr && (!MON || p.mon != nullptr) &&
-                          (!FO4 || (p.fo.S && p.fo.SMean && p.fo.k && p.fo.kMean)),
+                          (!FO4 || (p.fo.S && p.fo.SMean && p.fo.k && p.fo.kMean)) && (FO != 3 || p.fo.momentsMean),
                       CHK_PTR, 0);
     }
 #endif
@@ -767,7 +768,19 @@ __device__ __forceinline__ bool march_chunk(const CUtensorMap *tmap, const StepP
             });
             if (upd_node) {
                 const unsigned type = type_xy | (zu == 0 ? BACK : 0u) | (zu == p.nz - 1 ? FRONT : 0u);
-                float m[10];
+                float fold[10], m[10];
+                moment_folds<Q>(f, fold);
+                // The old means of the moments, all ten loads in flight at
+                // once (after the folds, when the populations' registers are
+                // free); read one by one at their update each waits for its
+                // own trip to memory: 248 us per step became 150 (D3Q27
+                // 136x120x128, all five function objects, FP64 means; 5.3 TB/s).
+                MeanT mm_old[10];
+                if constexpr (FO == 3) {
+#pragma unroll
+                    for (int c = 0; c < 10; c++)
+                        mm_old[c] = (p.fo.momentsMean + c * N)[iu];
+                }
                 if constexpr (CLM != 0) {
                     // interior nodes relax with tau0 + dtau; omega as the host
                     // derives it from tau, so dtau = 0 gives the plain bits
@@ -777,9 +790,9 @@ __device__ __forceinline__ bool march_chunk(const CUtensorMap *tmap, const StepP
                         r.t_omega = __fsub_rn(1.0f, r.omega);
                         r.omega_d2 = __fmul_rn(r.omega, 0.5f);
                     }
-                    node_update<Q>(f, type, r, m);
+                    node_update<Q>(fold, type, r, m);
                 } else {
-                    node_update<Q, Storage<ST>::SCI>(f, type, p.rx, m);
+                    node_update<Q, Storage<ST>::SCI>(fold, type, p.rx, m);
                 }
                 // m[1..9] come out of the collision scaled by SC, m[0] is rho
                 p.out[iu] = Storage<ST>::store_raw(stored_of_rho<ST>(m[0]));
@@ -820,13 +833,12 @@ __device__ __forceinline__ bool march_chunk(const CUtensorMap *tmap, const StepP
                         if (FO4 || p.fo.kMean)
                             p.fo.kMean[iu] = time_average<MeanT>(km_old, MeanT(ke), p.fo.inv_count);
                     }
-                    if (!FO4 && p.fo.momentsMean) {
+                    if constexpr (FO == 3) {
                         m[0] = m[0] - 1.0f;
 #pragma unroll
-                        for (int c = 0; c < 10; c++) {
-                            MeanT *a = p.fo.momentsMean + c * N + iu;  // (rare path)
-                            *a = time_average<MeanT>(*a, MeanT(m[c]), p.fo.inv_count);
-                        }
+                        for (int c = 0; c < 10; c++)
+                            (p.fo.momentsMean + c * N)[iu] =
+                                time_average<MeanT>(mm_old[c], MeanT(m[c]), p.fo.inv_count);
                     }
                 }
             }

@@ -45,15 +45,23 @@ void *kernel_fn()
 }
 
 // The function-object kernel for a set of function objects: none; exactly
-// S, SMean, k and kMean (code 2: no run-time checks); any other set (code 1).
+// S, SMean, k and kMean (code 2: no run-time checks); any set with momentsMean
+// (code 3); any other set (code 1).  Code 3 is apart because the old means of
+// the moments take ten registers (FP64: twenty) that the other sets' kernels
+// would spill for (D3Q19 256^3, k and kMean in FP64: 321 us per step alone,
+// 393 with them).
 constexpr unsigned kFoFour = 0x0Fu;  // LBM_FO_S | LBM_FO_SMEAN | LBM_FO_K | LBM_FO_KMEAN
+constexpr unsigned kFoMomentsMean = 0x10u;  // LBM_FO_MOMENTSMEAN
 
 template <int Q, int TX, int TY, int NS, int NPB, int MINB, typename ST, int FO>
 void pick_means(Launcher &l, int mean_bits)
 {
     if (mean_bits == 64) {
-        l.fn = kernel_fn<Q, TX, TY, NS, FO, double, false, NPB, MINB, ST>();
-        l.fn_mon = kernel_fn<Q, TX, TY, NS, FO, double, true, NPB, MINB, ST>();
+        // FP64 old means of all moments: 20 registers more are worth a CTA
+        // (256^3, all five: 1126 us per step at 3 CTAs/SM, 1058 at 2)
+        constexpr int MB = FO == 3 && MINB > 2 ? 2 : MINB;
+        l.fn = kernel_fn<Q, TX, TY, NS, FO, double, false, NPB, MB, ST>();
+        l.fn_mon = kernel_fn<Q, TX, TY, NS, FO, double, true, NPB, MB, ST>();
     } else {
         l.fn = kernel_fn<Q, TX, TY, NS, FO, float, false, NPB, MINB, ST>();
         l.fn_mon = kernel_fn<Q, TX, TY, NS, FO, float, true, NPB, MINB, ST>();
@@ -74,6 +82,8 @@ Launcher pick_fo(unsigned fo, int mean_bits)
         l.fn_mon = kernel_fn<Q, TX, TY, NS, 0, float, true, NPB, MINB, ST>();
     } else if (fo == kFoFour) {
         pick_means<Q, TX, TY, NS, NPB, MINB, ST, 2>(l, mean_bits);
+    } else if (fo & kFoMomentsMean) {
+        pick_means<Q, TX, TY, NS, NPB, MINB, ST, 3>(l, mean_bits);
     } else {
         pick_means<Q, TX, TY, NS, NPB, MINB, ST, 1>(l, mean_bits);
     }

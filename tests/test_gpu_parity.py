@@ -90,6 +90,26 @@ def test_default_shape_equals_a_named_one(q, shape, storage):
     assert bits_equal(out["moments"], base["moments"])
 
 
+@pytest.mark.parametrize("q,tile,npb", [(19, 32, 1), (19, 32, 4), (27, 32, 1), (27, 16, 1), (27, 8, 1)])
+@pytest.mark.parametrize("mean_bits", [32, 64])
+def test_function_object_kernels_agree(q, tile, npb, mean_bits):
+    """Sets of function objects run in different kernels; a field has the
+    same bits in all of them (the last tile partly outside the mesh)."""
+    four = ("S", "SMean", "k", "kMean")
+    base = None
+    for fo in (four + ("momentsMean",), four, ("momentsMean",), ("SMean", "momentsMean"), ("k", "kMean")):
+        with Cavity(q, 40, 16, 24, 400.0, 0.05, function_objects=fo, mean_bits=mean_bits, tile=(tile, 8, 2),
+                    pop_buffers=npb) as c:
+            c.init_regions()
+            c.perturb_velocity(1e-3, 5)
+            c.step(6)
+            out = {f: c.read(f, dtype=np.float64 if mean_bits == 64 and "Mean" in f else np.float32)
+                   for f in ("moments",) + fo}
+        base = base or out
+        for f in out:
+            assert out[f].tobytes() == base[f].tobytes(), (fo, f)
+
+
 @pytest.mark.parametrize("q", [19, 27])
 def test_against_fp64_oracle(q):
     n = (24, 16, 32)
