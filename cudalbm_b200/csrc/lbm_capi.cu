@@ -393,6 +393,23 @@ lbm_status ensure_scratch(lbm_handle *h, size_t bytes)
     return LBM_OK;
 }
 
+// Monitor slots for n steps.
+lbm_status ensure_mon_steps(lbm_handle *h, uint64_t n)
+{
+    if (h->mon_steps_cap >= n)
+        return LBM_OK;
+    if (h->mon_steps) {
+        cudaFree(h->mon_steps);
+        h->device_bytes -= h->mon_steps_cap * sizeof(lbm::MonitorSlot);
+        h->mon_steps = nullptr;
+        h->mon_steps_cap = 0;
+    }
+    LBM_CUDA(cudaMalloc(&h->mon_steps, n * sizeof(lbm::MonitorSlot)));
+    h->mon_steps_cap = n;
+    h->device_bytes += n * sizeof(lbm::MonitorSlot);
+    return LBM_OK;
+}
+
 // How one field set moves between host values and the device buffer.
 struct Xfer {
     size_t hsz;   // bytes per host value
@@ -524,11 +541,12 @@ bool means_f64(const lbm_handle *h)
     return h->cfg.function_objects != 0 && h->cfg.mean_bits == 64;
 }
 
+// One whole-mesh step; mon: the step's (zeroed) monitor slot, or null.
 template <typename MeanT>
-lbm_status launch_step(lbm_handle *h, bool monitored = false)
+lbm_status launch_step(lbm_handle *h, lbm::MonitorSlot *mon = nullptr)
 {
     if (h->closure) {
-        if (monitored)
+        if (mon)
             return fail(LBM_ERR_STATE, "monitored steps are not available with the learned closure");
         return lbm::closure_step(h);
     }
@@ -537,7 +555,7 @@ lbm_status launch_step(lbm_handle *h, bool monitored = false)
     StepParams<MeanT> p{};
     const int nxt = h->cur ^ 1;
     p.out = static_cast<float *>(h->m[nxt]);
-    p.mon = h->mon;
+    p.mon = mon;
     p.nx = int(h->cfg.nx);
     p.ny = int(h->cfg.ny);
     p.nz = int(h->cfg.nz);
@@ -571,7 +589,7 @@ lbm_status launch_step(lbm_handle *h, bool monitored = false)
                     unsigned((h->cfg.ny + h->launcher.ty - 1) / h->launcher.ty),
                     unsigned(zch.count));
     void *args[] = {&h->tmap[h->cur], &p};
-    LBM_CUDA(lbm::launch_overlapped(monitored ? h->launcher.fn_mon : h->launcher.fn, grid, block, args,
+    LBM_CUDA(lbm::launch_overlapped(mon ? h->launcher.fn_mon : h->launcher.fn, grid, block, args,
                                     h->launcher.smem, h->stream));
     h->cur = nxt;
     h->t += 1;
@@ -680,10 +698,12 @@ void destroy_handle(lbm_handle *h)
         cudaStreamSynchronize(h->stream);
     for (void *p : {h->m[0], h->m[1], static_cast<void *>(h->S), static_cast<void *>(h->k), h->SMean, h->kMean,
                     h->momentsMean, static_cast<void *>(h->err), static_cast<void *>(h->red),
-                    static_cast<void *>(h->mon), h->scratch, static_cast<void *>(h->dtau),
+                    h->scratch, static_cast<void *>(h->dtau),
                     static_cast<void *>(h->mon_steps)})
         if (p)
             cudaFree(p);
+    if (h->err_host)
+        cudaFreeHost(h->err_host);
     if (h->dstream) {
         cudaStreamSynchronize(h->dstream);
         cudaStreamDestroy(h->dstream);
@@ -839,8 +859,9 @@ lbm_status lbm_create(const lbm_config *cfg, lbm_handle **out)
     if (c.function_objects & LBM_FO_MOMENTSMEAN)
         if ((s = dev_alloc(h, reinterpret_cast<char **>(&h->momentsMean), 10 * h->N * msz)) != LBM_OK) return cleanup_fail(s);
     if ((s = dev_alloc(h, &h->err, 1)) != LBM_OK) return cleanup_fail(s);
+    if (cudaMallocHost(&h->err_host, sizeof(lbm::StepFault)) != cudaSuccess)
+        return cleanup_fail(fail(LBM_ERR_NOMEM, "cannot allocate page-locked host memory"));
     if ((s = dev_alloc(h, &h->red, 4)) != LBM_OK) return cleanup_fail(s);
-    if ((s = dev_alloc(h, &h->mon, 1)) != LBM_OK) return cleanup_fail(s);
     for (int b = 0; b < 2; b++) {
         cudaMemsetAsync(h->m[b], 0, 10 * h->N * h->esz, h->stream);
     }
@@ -1106,14 +1127,22 @@ lbm_status lbm_step_monitored(lbm_handle *h, uint64_t n, lbm_monitor *out)
     static_assert(sizeof(lbm_monitor) == sizeof(lbm::MonitorSlot), "monitor layout");
     if (n == 0)
         return LBM_OK;
+    // a slot per step, zeroed and copied to the host in blocks: with a memset
+    // and a copy around every step the steps cannot overlap
+    constexpr uint64_t kMonBlock = 4096;
+    lbm_status s = ensure_mon_steps(h, std::min(n, kMonBlock));
+    if (s != LBM_OK)
+        return s;
     LBM_CUDA(cudaEventRecord(h->ev0, h->stream));
     const bool md = means_f64(h);
-    for (uint64_t i = 0; i < n; i++) {
-        LBM_CUDA(cudaMemsetAsync(h->mon, 0, sizeof(lbm::MonitorSlot), h->stream));
-        lbm_status s = md ? launch_step<double>(h, true) : launch_step<float>(h, true);
-        if (s != LBM_OK)
-            return s;
-        LBM_CUDA(cudaMemcpyAsync(&out[i], h->mon, sizeof(lbm::MonitorSlot), cudaMemcpyDeviceToHost, h->stream));
+    for (uint64_t b = 0; b < n; b += kMonBlock) {
+        const uint64_t cnt = std::min(n - b, kMonBlock);
+        LBM_CUDA(cudaMemsetAsync(h->mon_steps, 0, cnt * sizeof(lbm::MonitorSlot), h->stream));
+        for (uint64_t i = 0; i < cnt; i++)
+            if ((s = md ? launch_step<double>(h, h->mon_steps + i) : launch_step<float>(h, h->mon_steps + i)) != LBM_OK)
+                return s;
+        LBM_CUDA(cudaMemcpyAsync(out + b, h->mon_steps, cnt * sizeof(lbm::MonitorSlot), cudaMemcpyDeviceToHost,
+                                 h->stream));
     }
     LBM_CUDA(cudaEventRecord(h->ev1, h->stream));
     h->timed = true;
@@ -1158,16 +1187,10 @@ lbm_status lbm_run_streamed(lbm_handle *h, const float *moments, uint64_t n, voi
         LBM_CUDA(cudaStreamCreateWithFlags(&h->xstream, cudaStreamNonBlocking));
     if (!h->dstream)
         LBM_CUDA(cudaStreamCreateWithFlags(&h->dstream, cudaStreamNonBlocking));
-    if (mon && h->mon_steps_cap < n) {
-        if (h->mon_steps) {
-            cudaFree(h->mon_steps);
-            h->device_bytes -= h->mon_steps_cap * sizeof(lbm::MonitorSlot);
-            h->mon_steps = nullptr;
-            h->mon_steps_cap = 0;
-        }
-        LBM_CUDA(cudaMalloc(&h->mon_steps, n * sizeof(lbm::MonitorSlot)));
-        h->mon_steps_cap = n;
-        h->device_bytes += n * sizeof(lbm::MonitorSlot);
+    if (mon) {
+        lbm_status ms = ensure_mon_steps(h, n);
+        if (ms != LBM_OK)
+            return ms;
     }
     const int nz = int(h->cfg.nz);
     const size_t plane = size_t(h->cfg.nx) * size_t(h->cfg.ny);
@@ -1379,10 +1402,11 @@ lbm_status lbm_synchronize(lbm_handle *h)
     if (!h)
         return fail(LBM_ERR_ARG, "null handle");
     LBM_CUDA(cudaSetDevice(h->cfg.device));
+    // the record arrives with the queued work: one wait instead of a wait and
+    // a blocking copy
+    LBM_CUDA(cudaMemcpyAsync(h->err_host, h->err, sizeof(lbm::StepFault), cudaMemcpyDeviceToHost, h->stream));
     LBM_CUDA(cudaStreamSynchronize(h->stream));
-    lbm::StepFault f{};
-    LBM_CUDA(cudaMemcpy(&f, h->err, sizeof(f), cudaMemcpyDeviceToHost));
-    return lbm::check_fault(f, "a step kernel");
+    return lbm::check_fault(*h->err_host, "a step kernel");
 }
 
 lbm_status lbm_reduce(lbm_handle *h, double out[3])

@@ -31,6 +31,7 @@ struct lbm_handle {
     float *S = nullptr, *k = nullptr;
     void *SMean = nullptr, *kMean = nullptr, *momentsMean = nullptr;
     lbm::StepFault *err = nullptr;    // device-side error record of the step kernels
+    lbm::StepFault *err_host = nullptr;  // page-locked copy of it (lbm_synchronize)
     double *red = nullptr;
     void *scratch = nullptr;
     size_t scratch_bytes = 0;
@@ -40,10 +41,9 @@ struct lbm_handle {
     cudaStream_t xstream = nullptr;
     cudaEvent_t xe_copied[2] = {nullptr, nullptr};
     cudaEvent_t xe_converted[2] = {nullptr, nullptr};
-    // lbm_run_streamed: uploads go on xstream, downloads on dstream; one
-    // monitor slot per step of the job
+    // lbm_run_streamed: uploads go on xstream, downloads on dstream
     cudaStream_t dstream = nullptr;
-    lbm::MonitorSlot *mon_steps = nullptr;
+    lbm::MonitorSlot *mon_steps = nullptr;  // a slot per monitored step of a call (or of a block of its steps)
     size_t mon_steps_cap = 0;
     float tau = 0, omega = 0, t_omega = 0, omega_d2 = 0;
     int64_t t = 0;
@@ -53,7 +53,6 @@ struct lbm_handle {
     uint64_t launches = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     bool timed = false;
-    lbm::MonitorSlot *mon = nullptr;  // one slot, reused by every monitored step
     // learned closure (lbm_closure.cu)
     bool closure = false;
     float *dtau = nullptr;             // [N] relaxation-time correction of the current step

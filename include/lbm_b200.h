@@ -147,7 +147,7 @@ typedef struct lbm_monitor {
 } lbm_monitor;
 
 /* lbm_step with a per-step result: step i writes its sums to out[i] (n
- * entries) by an asynchronous device-to-host copy queued after the step.
+ * entries); an asynchronous device-to-host copy follows the steps (every 4096).
  * With page-locked `out` (lbm_host_alloc) nothing waits for the host; the
  * values are valid after lbm_synchronize.  Replaces: the reference's per-step
  * info print (momentBasedD3Q19.cu:107-110) and fieldCalculate containsNaN
