@@ -50,6 +50,18 @@ def test_statistics_match_the_oracle(shape, tiled):
     assert np.all(nan == 0)
 
 
+@pytest.mark.parametrize("shape", [(1, 1, 1), (3, 5, 7), (5, 1, 63), (1, 1, 64), (2, 33, 62), (1, 17, 241),
+                                   (97, 113, 251)])
+def test_ordered_sum_at_chunk_and_slice_edges(shape):
+    """One value, less and more than the values read ahead, one chunk short
+    of and past 4096 values, and several slices of a mesh of odd edges."""
+    f = random_fields(shape, nf=3, seed=11)
+    nan, mean_ref, mean = field_statistics(f)
+    ref = np.array([fo.spatial_mean(x) for x in f], np.float32)
+    assert np.array_equal(mean_ref.view(np.uint32), ref.view(np.uint32))
+    assert np.allclose(mean, f.reshape(3, -1).astype(np.float64).mean(axis=1), rtol=1e-12, atol=1e-15)
+
+
 def test_nan_counts_and_infinities():
     shape = (24, 16, 32)
     f = random_fields(shape, nf=5, seed=3)
