@@ -702,8 +702,6 @@ void destroy_handle(lbm_handle *h)
                     static_cast<void *>(h->mon_steps)})
         if (p)
             cudaFree(p);
-    if (h->err_host)
-        cudaFreeHost(h->err_host);
     if (h->dstream) {
         cudaStreamSynchronize(h->dstream);
         cudaStreamDestroy(h->dstream);
@@ -859,8 +857,6 @@ lbm_status lbm_create(const lbm_config *cfg, lbm_handle **out)
     if (c.function_objects & LBM_FO_MOMENTSMEAN)
         if ((s = dev_alloc(h, reinterpret_cast<char **>(&h->momentsMean), 10 * h->N * msz)) != LBM_OK) return cleanup_fail(s);
     if ((s = dev_alloc(h, &h->err, 1)) != LBM_OK) return cleanup_fail(s);
-    if (cudaMallocHost(&h->err_host, sizeof(lbm::StepFault)) != cudaSuccess)
-        return cleanup_fail(fail(LBM_ERR_NOMEM, "cannot allocate page-locked host memory"));
     if ((s = dev_alloc(h, &h->red, 4)) != LBM_OK) return cleanup_fail(s);
     for (int b = 0; b < 2; b++) {
         cudaMemsetAsync(h->m[b], 0, 10 * h->N * h->esz, h->stream);
@@ -1402,11 +1398,12 @@ lbm_status lbm_synchronize(lbm_handle *h)
     if (!h)
         return fail(LBM_ERR_ARG, "null handle");
     LBM_CUDA(cudaSetDevice(h->cfg.device));
-    // the record arrives with the queued work: one wait instead of a wait and
-    // a blocking copy
-    LBM_CUDA(cudaMemcpyAsync(h->err_host, h->err, sizeof(lbm::StepFault), cudaMemcpyDeviceToHost, h->stream));
+    // the record is copied in the order of the stream: one wait instead of a
+    // wait and a blocking copy on another stream
+    lbm::StepFault f{};
+    LBM_CUDA(cudaMemcpyAsync(&f, h->err, sizeof(f), cudaMemcpyDeviceToHost, h->stream));
     LBM_CUDA(cudaStreamSynchronize(h->stream));
-    return lbm::check_fault(*h->err_host, "a step kernel");
+    return lbm::check_fault(f, "a step kernel");
 }
 
 lbm_status lbm_reduce(lbm_handle *h, double out[3])

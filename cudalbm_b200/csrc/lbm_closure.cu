@@ -252,110 +252,212 @@ __global__ void __launch_bounds__(kSampleCta) write_samples_kernel(TargetArgs a,
 }
 
 // ----------------------------------------------------- training kernels
-// d gelu / dz of the tanh form
-__device__ __forceinline__ float gelu_grad(float z)
+// gelu(z) of the tanh form and its derivative
+__device__ __forceinline__ void gelu_and_grad(float z, float &h, float &dh)
 {
     const float t = tanhf(lbm::kGeluA * fmaf(lbm::kGeluB * z * z, z, z));
-    return 0.5f * (1.0f + t) + 0.5f * z * (1.0f - t * t) * lbm::kGeluA * fmaf(3.0f * lbm::kGeluB, z * z, 1.0f);
+    h = 0.5f * z * (1.0f + t);
+    dh = 0.5f * (1.0f + t) + 0.5f * z * (1.0f - t * t) * lbm::kGeluA * fmaf(3.0f * lbm::kGeluB, z * z, 1.0f);
 }
 
 // Mean squared error gradient over a batch.  Sample s of the batch is
-// first + s (sequential) or hash(seed, s) % n (random).  Phase 1: one thread
-// per sample, forward and backward, per-sample factors into shared memory;
-// phase 2: one thread per parameter sums its products over the CTA's samples
-// and adds them to grad (FP32 atomics).
-constexpr int kTrainCta = 128;
+// first + s (sequential) or hash(seed, s) % n (random).  A CTA takes 128
+// samples with four threads each: a thread computes 8 of a layer's 32 units
+// (warps hold one part of 32 samples, so weights are broadcast and the
+// [unit][sample] arrays are read without conflicts); then the threads share
+// the parameters, 2x2 tiles of w2 and w1 and single biases, and sum their
+// products over the CTA's samples in order.  What bounds it is a chain: few
+// CTAs (64 for a batch of 8192), each of dependent layers.  8192 samples: 16
+// us; one thread per sample and one parameter at a time took 46 (and 17
+// instead of 64 us per Adam step with reduce_adam_kernel and the overlapped
+// launches).  The sums keep that order.
+constexpr int kTrainCta = 128, kTrainParts = 4, kTrainThreads = kTrainCta * kTrainParts;
+constexpr int kUnits = kMlpHidden / kTrainParts, kRow = kTrainCta + 1;
 struct TrainSmem {
     MlpParams p;
-    float xs[kTrainCta][kMlpIn];
-    float h1[kTrainCta][kMlpHidden], h2[kTrainCta][kMlpHidden];
-    float dz1[kTrainCta][kMlpHidden], dz2[kTrainCta][kMlpHidden];
+    float xs[kMlpIn][kRow];
+    float h1[kMlpHidden][kRow], h2[kMlpHidden][kRow];
+    float dz1[kMlpHidden][kRow], dz2[kMlpHidden][kRow];
     float dy[kTrainCta];
 };
+static_assert(offsetof(MlpParams, w2) % 16 == 0 && offsetof(MlpParams, w1) % 16 == 0, "weights are read 16 bytes at a time");
 
-__global__ void __launch_bounds__(kTrainCta) grad_kernel(const float *feat, const float *targ, uint64_t n,
-                                                         uint64_t first, uint64_t batch, uint64_t seed, int random,
-                                                         const MlpParams *params, float *partial, double *loss_partial)
+__global__ void __launch_bounds__(kTrainThreads) grad_kernel(const float *feat, const float *targ, uint64_t n,
+                                                             uint64_t first, uint64_t batch, uint64_t seed, int random,
+                                                             const MlpParams *params, float *partial,
+                                                             double *loss_partial)
 {
     extern __shared__ __align__(16) unsigned char raw[];
     TrainSmem &S = *reinterpret_cast<TrainSmem *>(raw);
-    const int t = threadIdx.x;
-    for (int i = t; i < int(sizeof(MlpParams) / 4); i += kTrainCta)
+    const int t = threadIdx.x, r = t & (kTrainCta - 1), part = t / kTrainCta, u0 = part * kUnits;
+    const uint64_t s = uint64_t(blockIdx.x) * kTrainCta + r;
+    const bool valid = s < batch;
+    lbm::let_next_grid_start();
+    // this sample's features 4 part .. 4 part + 3 and target; the samples are
+    // not written by the kernels in front of this one
+    static_assert(kMlpIn == 4 * kTrainParts, "four features per thread");
+    float4 fv = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float target = 0.0f;
+    if (valid) {
+        const uint64_t idx = random ? splitmix64(seed ^ (s * 0xD6E8FEB86659FD93ull)) % n : first + s;
+        fv = *reinterpret_cast<const float4 *>(feat + idx * kMlpIn + 4 * part);
+        target = targ[idx];
+    }
+    lbm::wait_previous_grid();
+    for (int i = t; i < int(sizeof(MlpParams) / 4); i += kTrainThreads)
         reinterpret_cast<float *>(&S.p)[i] = reinterpret_cast<const float *>(params)[i];
     __syncthreads();
-    const uint64_t s = uint64_t(blockIdx.x) * kTrainCta + t;
-    float xs[kMlpIn], z1[kMlpHidden], h1[kMlpHidden], z2[kMlpHidden], h2[kMlpHidden];
-    float dy = 0.0f, e2 = 0.0f;
-    if (s < batch) {
-        const uint64_t idx = random ? splitmix64(seed ^ (s * 0xD6E8FEB86659FD93ull)) % n : first + s;
+    {
+        const float f[4] = {fv.x, fv.y, fv.z, fv.w};
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const int k = 4 * part + c;
+            S.xs[k][r] = valid ? (f[c] - S.p.in_mean[k]) * S.p.in_scale[k] : 0.0f;
+        }
+    }
+    __syncthreads();
+    float g1[kUnits], g2[kUnits];  // derivatives of the activations
+    {
+        float x[kMlpIn];
+#pragma unroll
         for (int k = 0; k < kMlpIn; k++)
-            xs[k] = (feat[idx * kMlpIn + k] - S.p.in_mean[k]) * S.p.in_scale[k];
-        const float y = lbm::mlp_forward_f32(S.p, xs, z1, h1, z2, h2);
-        const float ts = fminf(fmaxf(targ[idx], S.p.dtau_lo), S.p.dtau_hi) / S.p.out_scale;
+            x[k] = S.xs[k][r];
+#pragma unroll
+        for (int u = 0; u < kUnits; u++) {
+            float a = S.p.b1[u0 + u], h;
+            const float4 *w = reinterpret_cast<const float4 *>(S.p.w1 + (u0 + u) * kMlpIn);
+#pragma unroll
+            for (int k = 0; k < kMlpIn / 4; k++) {
+                const float4 q = w[k];
+                a = fmaf(q.x, x[4 * k], a);
+                a = fmaf(q.y, x[4 * k + 1], a);
+                a = fmaf(q.z, x[4 * k + 2], a);
+                a = fmaf(q.w, x[4 * k + 3], a);
+            }
+            gelu_and_grad(a, h, g1[u]);
+            S.h1[u0 + u][r] = valid ? h : 0.0f;
+        }
+    }
+    __syncthreads();
+    {
+        float x[kMlpHidden];
+#pragma unroll
+        for (int k = 0; k < kMlpHidden; k++)
+            x[k] = S.h1[k][r];
+#pragma unroll
+        for (int u = 0; u < kUnits; u++) {
+            float a = S.p.b2[u0 + u], h;
+            const float4 *w = reinterpret_cast<const float4 *>(S.p.w2 + (u0 + u) * kMlpHidden);
+#pragma unroll
+            for (int k = 0; k < kMlpHidden / 4; k++) {
+                const float4 q = w[k];
+                a = fmaf(q.x, x[4 * k], a);
+                a = fmaf(q.y, x[4 * k + 1], a);
+                a = fmaf(q.z, x[4 * k + 2], a);
+                a = fmaf(q.w, x[4 * k + 3], a);
+            }
+            gelu_and_grad(a, h, g2[u]);
+            S.h2[u0 + u][r] = valid ? h : 0.0f;
+        }
+    }
+    __syncthreads();
+    // output and error (every part for itself)
+    float dy = 0.0f, e2 = 0.0f;
+    if (valid) {
+        float y = S.p.b3;
+#pragma unroll
+        for (int j = 0; j < kMlpHidden; j++)
+            y = fmaf(S.p.w3[j], S.h2[j][r], y);
+        const float ts = fminf(fmaxf(target, S.p.dtau_lo), S.p.dtau_hi) / S.p.out_scale;
         const float e = y - ts;
         e2 = e * e;
         dy = 2.0f * e / float(batch);
-    } else {
-        for (int k = 0; k < kMlpIn; k++)
-            xs[k] = 0.0f;
-        for (int j = 0; j < kMlpHidden; j++)
-            z1[j] = h1[j] = z2[j] = h2[j] = 0.0f;
     }
-    float dz2[kMlpHidden];
-    for (int j = 0; j < kMlpHidden; j++)
-        dz2[j] = dy * S.p.w3[j] * gelu_grad(z2[j]);
-    for (int k = 0; k < kMlpHidden; k++) {
-        float a = 0.0f;
-        for (int j = 0; j < kMlpHidden; j++)
-            a = fmaf(dz2[j], S.p.w2[j * kMlpHidden + k], a);
-        S.dz1[t][k] = a * gelu_grad(z1[k]);
-        S.h1[t][k] = h1[k];
-        S.h2[t][k] = h2[k];
-        S.dz2[t][k] = dz2[k];
-    }
-    for (int k = 0; k < kMlpIn; k++)
-        S.xs[t][k] = xs[k];
-    S.dy[t] = dy;
+#pragma unroll
+    for (int u = 0; u < kUnits; u++)
+        S.dz2[u0 + u][r] = dy * S.p.w3[u0 + u] * g2[u];
     // CTA sum of the squared errors, in a fixed order
-    double e2d = double(e2);
-    for (int o = 16; o > 0; o >>= 1)
-        e2d += __shfl_down_sync(0xffffffffu, e2d, o);
     __shared__ double warp_e2[kTrainCta / 32];
-    if ((t & 31) == 0)
-        warp_e2[t >> 5] = e2d;
+    if (part == 0) {
+        S.dy[r] = dy;
+        double e2d = double(e2);
+        for (int o = 16; o > 0; o >>= 1)
+            e2d += __shfl_down_sync(0xffffffffu, e2d, o);
+        if ((t & 31) == 0)
+            warp_e2[t >> 5] = e2d;
+    }
     __syncthreads();
+    {
+        float a[kUnits] = {};
+#pragma unroll 8
+        for (int j = 0; j < kMlpHidden; j++) {
+            const float d = S.dz2[j][r];
+            const float4 *w = reinterpret_cast<const float4 *>(S.p.w2 + j * kMlpHidden + u0);
+#pragma unroll
+            for (int k = 0; k < kUnits / 4; k++) {
+                const float4 q = w[k];
+                a[4 * k] = fmaf(d, q.x, a[4 * k]);
+                a[4 * k + 1] = fmaf(d, q.y, a[4 * k + 1]);
+                a[4 * k + 2] = fmaf(d, q.z, a[4 * k + 2]);
+                a[4 * k + 3] = fmaf(d, q.w, a[4 * k + 3]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kUnits; u++)
+            S.dz1[u0 + u][r] = a[u] * g1[u];
+    }
     if (t == 0) {
         double sum = 0.0;
         for (int w = 0; w < kTrainCta / 32; w++)
             sum += warp_e2[w];
         loss_partial[blockIdx.x] = sum;
     }
-    // phase 2: parameter p (the lbm_mlp weight order w1, b1, w2, b2, w3, b3)
-    for (int p = t; p < kMlpWeights; p += kTrainCta) {
-        float acc = 0.0f;
-        int q = p;
-        if (q < kMlpHidden * kMlpIn) {
-            const int j = q / kMlpIn, i = q % kMlpIn;
-            for (int r = 0; r < kTrainCta; r++)
-                acc = fmaf(S.dz1[r][j], S.xs[r][i], acc);
-        } else if ((q -= kMlpHidden * kMlpIn) < kMlpHidden) {
-            for (int r = 0; r < kTrainCta; r++)
-                acc += S.dz1[r][q];
-        } else if ((q -= kMlpHidden) < kMlpHidden * kMlpHidden) {
-            const int j = q / kMlpHidden, k = q % kMlpHidden;
-            for (int r = 0; r < kTrainCta; r++)
-                acc = fmaf(S.dz2[r][j], S.h1[r][k], acc);
-        } else if ((q -= kMlpHidden * kMlpHidden) < kMlpHidden) {
-            for (int r = 0; r < kTrainCta; r++)
-                acc += S.dz2[r][q];
-        } else if ((q -= kMlpHidden) < kMlpHidden) {
-            for (int r = 0; r < kTrainCta; r++)
-                acc = fmaf(S.dy[r], S.h2[r][q], acc);
-        } else {
-            for (int r = 0; r < kTrainCta; r++)
-                acc += S.dy[r];
+    __syncthreads();
+    // parameter gradients (the lbm_mlp weight order w1, b1, w2, b2, w3, b3)
+    float *const out = partial + size_t(blockIdx.x) * kMlpWeights;
+    constexpr int kB1 = kMlpHidden * kMlpIn, kW2 = kB1 + kMlpHidden, kB2 = kW2 + kMlpHidden * kMlpHidden,
+                  kW3 = kB2 + kMlpHidden, kB3 = kW3 + kMlpHidden;
+    constexpr int kTiles2 = (kMlpHidden / 2) * (kMlpHidden / 2), kTiles1 = (kMlpHidden / 2) * (kMlpIn / 2);
+    static_assert(kTiles2 + kTiles1 + 3 * kMlpHidden + 1 <= kTrainThreads && kB3 + 1 == kMlpWeights, "one round");
+    auto tile = [&](const float *d0, const float *d1, const float *x0, const float *x1, float *g, int row) {
+        float a00 = 0.0f, a01 = 0.0f, a10 = 0.0f, a11 = 0.0f;
+#pragma unroll 8
+        for (int i = 0; i < kTrainCta; i++) {
+            a00 = fmaf(d0[i], x0[i], a00);
+            a01 = fmaf(d0[i], x1[i], a01);
+            a10 = fmaf(d1[i], x0[i], a10);
+            a11 = fmaf(d1[i], x1[i], a11);
         }
-        partial[size_t(blockIdx.x) * kMlpWeights + p] = acc;
+        g[0] = a00;
+        g[1] = a01;
+        g[row] = a10;
+        g[row + 1] = a11;
+    };
+    if (t < kTiles2) {
+        const int j = t / (kMlpHidden / 2) * 2, k = t % (kMlpHidden / 2) * 2;
+        tile(S.dz2[j], S.dz2[j + 1], S.h1[k], S.h1[k + 1], out + kW2 + j * kMlpHidden + k, kMlpHidden);
+    } else if (t < kTiles2 + kTiles1) {
+        const int q = t - kTiles2, j = q / (kMlpIn / 2) * 2, k = q % (kMlpIn / 2) * 2;
+        tile(S.dz1[j], S.dz1[j + 1], S.xs[k], S.xs[k + 1], out + j * kMlpIn + k, kMlpIn);
+    } else {
+        const int q = t - kTiles2 - kTiles1, k = q % kMlpHidden;
+        float acc = 0.0f;
+        if (q < 2 * kMlpHidden) {
+            const float *d = q < kMlpHidden ? S.dz1[k] : S.dz2[k];
+#pragma unroll 8
+            for (int i = 0; i < kTrainCta; i++)
+                acc += d[i];
+            out[(q < kMlpHidden ? kB1 : kB2) + k] = acc;
+        } else if (q < 3 * kMlpHidden) {
+#pragma unroll 8
+            for (int i = 0; i < kTrainCta; i++)
+                acc = fmaf(S.dy[i], S.h2[k][i], acc);
+            out[kW3 + k] = acc;
+        } else if (q == 3 * kMlpHidden) {
+            for (int i = 0; i < kTrainCta; i++)
+                acc += S.dy[i];
+            out[kB3] = acc;
+        }
     }
 }
 
@@ -378,15 +480,33 @@ __global__ void reduce_partials_kernel(const float *partial, const double *loss_
     }
 }
 
-// Adam (Kingma & Ba 2015) over the kMlpWeights leading floats of MlpParams.
-__global__ void adam_kernel(float *w, const float *g, float *m, float *v, float lr, float c1, float c2)
+// The CTAs' partial gradients summed in CTA order, then Adam (Kingma & Ba
+// 2015) over the kMlpWeights leading floats of MlpParams; the thread after the
+// last parameter sums the losses.
+constexpr int kAdamCta = 64;
+__global__ void __launch_bounds__(kAdamCta) reduce_adam_kernel(const float *partial, const double *loss_partial,
+                                                               int ctas, float *w, float *m, float *v, double *loss,
+                                                               float lr, float c1, float c2)
 {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    const int p = blockIdx.x * kAdamCta + threadIdx.x;
+    lbm::let_next_grid_start();
+    lbm::wait_previous_grid();
+    if (p == kMlpWeights) {
+        double l = 0.0;
+#pragma unroll 16
+        for (int b = 0; b < ctas; b++)
+            l += loss_partial[b];
+        *loss = l;
+    }
     if (p >= kMlpWeights)
         return;
+    float g = 0.0f;
+#pragma unroll 16
+    for (int b = 0; b < ctas; b++)
+        g += partial[size_t(b) * kMlpWeights + p];
     const float b1 = 0.9f, b2 = 0.999f;
-    m[p] = b1 * m[p] + (1.0f - b1) * g[p];
-    v[p] = b2 * v[p] + (1.0f - b2) * g[p] * g[p];
+    m[p] = b1 * m[p] + (1.0f - b1) * g;
+    v[p] = b2 * v[p] + (1.0f - b2) * g * g;
     w[p] -= lr * (m[p] * c1) / (sqrtf(v[p] * c2) + 1e-8f);
 }
 
@@ -913,7 +1033,7 @@ lbm_status lbm_trainer_gradient(lbm_trainer *t, const lbm_mlp *net, uint64_t fir
     }
     cudaMemcpy(dp, net, sizeof(MlpParams), cudaMemcpyHostToDevice);
     cudaFuncSetAttribute(grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(TrainSmem)));
-    grad_kernel<<<ctas, kTrainCta, sizeof(TrainSmem), t->stream>>>(t->feat, t->targ, n, first, count, 0, 0, dp,
+    grad_kernel<<<ctas, kTrainThreads, sizeof(TrainSmem), t->stream>>>(t->feat, t->targ, n, first, count, 0, 0, dp,
                                                                    dpart, dlpart);
     reduce_partials_kernel<<<(kMlpWeights + 255) / 256, 256, 0, t->stream>>>(dpart, dlpart, int(ctas), dg, dl);
     cudaError_t e = cudaGetLastError();
@@ -951,21 +1071,24 @@ lbm_status lbm_trainer_fit(lbm_trainer *t, const lbm_train_options *opt, lbm_mlp
     if ((s = lbm_trainer_samples(t, 0, n, F.data(), T.data(), nullptr)) != LBM_OK)
         return s;
     MlpParams P{};
-    for (int k = 0; k < kMlpIn; k++) {
-        double sum = 0.0, sq = 0.0;
-        float lo = F[k], hi = F[k];
-        for (uint64_t i = 0; i < n; i++) {
-            const double v = F[i * kMlpIn + k];
-            sum += v;
-            sq += v * v;
-            lo = std::min(lo, F[i * kMlpIn + k]);
-            hi = std::max(hi, F[i * kMlpIn + k]);
+    {
+        // sample by sample, so that the 16 features' sums advance together
+        double sum[kMlpIn] = {}, sq[kMlpIn] = {};
+        std::copy_n(F.begin(), kMlpIn, P.in_lo);
+        std::copy_n(F.begin(), kMlpIn, P.in_hi);
+        for (uint64_t i = 0; i < n; i++)
+            for (int k = 0; k < kMlpIn; k++) {
+                const float f = F[i * kMlpIn + k];
+                sum[k] += double(f);
+                sq[k] += double(f) * double(f);
+                P.in_lo[k] = std::min(P.in_lo[k], f);
+                P.in_hi[k] = std::max(P.in_hi[k], f);
+            }
+        for (int k = 0; k < kMlpIn; k++) {
+            const double mean = sum[k] / double(n), var = std::max(sq[k] / double(n) - mean * mean, 0.0);
+            P.in_mean[k] = float(mean);
+            P.in_scale[k] = var > 0.0 ? float(1.0 / std::sqrt(var)) : 1.0f;
         }
-        const double mean = sum / double(n), var = std::max(sq / double(n) - mean * mean, 0.0);
-        P.in_mean[k] = float(mean);
-        P.in_scale[k] = var > 0.0 ? float(1.0 / std::sqrt(var)) : 1.0f;
-        P.in_lo[k] = lo;
-        P.in_hi[k] = hi;
     }
     double tsum = 0.0, tsq = 0.0;
     for (uint64_t i = 0; i < n; i++) {
@@ -992,20 +1115,18 @@ lbm_status lbm_trainer_fit(lbm_trainer *t, const lbm_train_options *opt, lbm_mlp
     const uint64_t B = uint64_t(opt->batch);
     const unsigned blocks = unsigned((B + kTrainCta - 1) / kTrainCta);
     MlpParams *dp = nullptr;
-    float *dg = nullptr, *dm = nullptr, *dv = nullptr, *dpart = nullptr;
+    float *dm = nullptr, *dv = nullptr, *dpart = nullptr;
     double *dl = nullptr, *dlpart = nullptr;
     auto release = [&]() {
         cudaFree(dp);
-        cudaFree(dg);
         cudaFree(dm);
         cudaFree(dv);
         cudaFree(dl);
         cudaFree(dpart);
         cudaFree(dlpart);
     };
-    if (cudaMalloc(&dp, sizeof(MlpParams)) != cudaSuccess || cudaMalloc(&dg, kMlpWeights * 4) != cudaSuccess ||
-        cudaMalloc(&dm, kMlpWeights * 4) != cudaSuccess || cudaMalloc(&dv, kMlpWeights * 4) != cudaSuccess ||
-        cudaMalloc(&dl, sizeof(double)) != cudaSuccess ||
+    if (cudaMalloc(&dp, sizeof(MlpParams)) != cudaSuccess || cudaMalloc(&dm, kMlpWeights * 4) != cudaSuccess || cudaMalloc(&dv, kMlpWeights * 4) != cudaSuccess ||
+        cudaMalloc(&dl, size_t(opt->steps) * sizeof(double)) != cudaSuccess ||
         cudaMalloc(&dpart, size_t(blocks) * kMlpWeights * 4) != cudaSuccess ||
         cudaMalloc(&dlpart, blocks * sizeof(double)) != cudaSuccess) {
         release();
@@ -1015,23 +1136,35 @@ lbm_status lbm_trainer_fit(lbm_trainer *t, const lbm_train_options *opt, lbm_mlp
     cudaMemset(dm, 0, kMlpWeights * 4);
     cudaMemset(dv, 0, kMlpWeights * 4);
     cudaFuncSetAttribute(grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(TrainSmem)));
-    double first_loss = -1.0, last_loss = 0.0;
     const int window = std::max(1, std::min(opt->steps / 10, 100));
-    double acc = 0.0;
+    cudaError_t e = cudaSuccess;
+    for (int step = 0; step < opt->steps && e == cudaSuccess; step++) {
+        uint64_t first = 0, seed = splitmix64(opt->seed + 0x51ED27ull * uint64_t(step + 1));
+        int random = 1, ctas = int(blocks);
+        double *loss = dl + step;
+        float c1 = 1.0f / (1.0f - std::pow(0.9f, float(step + 1))), c2 = 1.0f / (1.0f - std::pow(0.999f, float(step + 1)));
+        float lr = opt->lr, *w = reinterpret_cast<float *>(dp);
+        uint64_t batch = B;
+        void *ga[] = {&t->feat, &t->targ, &n, &first, &batch, &seed, &random, &dp, &dpart, &dlpart};
+        void *aa[] = {&dpart, &dlpart, &ctas, &w, &dm, &dv, &loss, &lr, &c1, &c2};
+        e = lbm::launch_overlapped(reinterpret_cast<const void *>(&grad_kernel), dim3(blocks), dim3(kTrainThreads), ga,
+                                   sizeof(TrainSmem), t->stream);
+        if (e == cudaSuccess)
+            e = lbm::launch_overlapped(reinterpret_cast<const void *>(&reduce_adam_kernel),
+                                       dim3(kMlpWeights / kAdamCta + 1), dim3(kAdamCta), aa, 0, t->stream);
+    }
+    // every step's loss, read once at the end
+    std::vector<double> losses(size_t(opt->steps));
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(losses.data(), dl, losses.size() * sizeof(double), cudaMemcpyDeviceToHost, t->stream);
+    const cudaError_t es = cudaStreamSynchronize(t->stream);
+    if (e == cudaSuccess)
+        e = es;
+    double first_loss = -1.0, last_loss = 0.0, acc = 0.0;
     int acc_n = 0;
-    for (int step = 0; step < opt->steps; step++) {
-        grad_kernel<<<blocks, kTrainCta, sizeof(TrainSmem), t->stream>>>(
-            t->feat, t->targ, n, 0, B, splitmix64(opt->seed + 0x51ED27ull * uint64_t(step + 1)), 1, dp, dpart, dlpart);
-        reduce_partials_kernel<<<(kMlpWeights + 255) / 256, 256, 0, t->stream>>>(dpart, dlpart, int(blocks), dg, dl);
-        const float c1 = 1.0f / (1.0f - std::pow(0.9f, float(step + 1)));
-        const float c2 = 1.0f / (1.0f - std::pow(0.999f, float(step + 1)));
-        adam_kernel<<<(kMlpWeights + 255) / 256, 256, 0, t->stream>>>(reinterpret_cast<float *>(dp), dg, dm, dv,
-                                                                       opt->lr, c1, c2);
+    for (int step = 0; step < opt->steps; step++)
         if (step < window || step >= opt->steps - window) {
-            double l = 0.0;
-            cudaMemcpyAsync(&l, dl, sizeof(double), cudaMemcpyDeviceToHost, t->stream);
-            cudaStreamSynchronize(t->stream);
-            acc += l / double(B);
+            acc += losses[size_t(step)] / double(B);
             if (++acc_n == window) {
                 if (first_loss < 0.0)
                     first_loss = acc / window;
@@ -1041,10 +1174,6 @@ lbm_status lbm_trainer_fit(lbm_trainer *t, const lbm_train_options *opt, lbm_mlp
                 acc_n = 0;
             }
         }
-    }
-    cudaError_t e = cudaStreamSynchronize(t->stream);
-    if (e == cudaSuccess)
-        e = cudaGetLastError();
     if (e == cudaSuccess)
         e = cudaMemcpy(&P, dp, sizeof(P), cudaMemcpyDeviceToHost);
     release();

@@ -31,7 +31,6 @@ struct lbm_handle {
     float *S = nullptr, *k = nullptr;
     void *SMean = nullptr, *kMean = nullptr, *momentsMean = nullptr;
     lbm::StepFault *err = nullptr;    // device-side error record of the step kernels
-    lbm::StepFault *err_host = nullptr;  // page-locked copy of it (lbm_synchronize)
     double *red = nullptr;
     void *scratch = nullptr;
     size_t scratch_bytes = 0;

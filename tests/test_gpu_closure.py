@@ -88,6 +88,20 @@ def test_gradient_matches_fp64_oracle(samples):
         assert np.linalg.norm(a - b) <= 2e-4 * np.linalg.norm(b) + 1e-12, name
 
 
+@pytest.mark.parametrize("count", [1, 31, 127, 128, 129])
+def test_gradient_at_the_edges_of_a_cta(samples, count):
+    """One sample, a warp not full, one short of, all and past a CTA's 128."""
+    tr, feats, targ, _, _ = samples
+    net = random_net(feats, targ, seed=4)
+    g, loss = tr.gradient(net, 3, count)
+    ref, ref_loss = mo.gradient(mo.params_of(net), feats[3:3 + count], targ[3:3 + count])
+    assert abs(loss - ref_loss) <= 1e-4 * ref_loss
+    gp = mo.params_of(g)
+    for name in mo.WEIGHTS:
+        a, b = np.ravel(gp[name]), np.ravel(ref[name])
+        assert np.linalg.norm(a - b) <= 2e-4 * np.linalg.norm(b) + 1e-12, name
+
+
 def test_inference_tensor_cores_and_fp32_paths(samples):
     _, feats, targ, _, _ = samples
     net = random_net(feats, targ, seed=3, scale=0.5)
