@@ -222,11 +222,10 @@ struct Relax {
     float omega, t_omega, omega_d2, tau, u_lid;
 };
 
-// Interior moments (unscaled) from the folds: velocitySet.cuh:398-417.
-__device__ __forceinline__ void interior_moments(const float *s, float *mom)
+// Interior moments (unscaled) from the folds and 1 / s[0]: velocitySet.cuh:398-417.
+__device__ __forceinline__ void interior_moments(const float *s, float inv_rho, float *mom)
 {
     mom[0] = s[0];
-    const float inv_rho = 1.0f / mom[0];
     mom[1] = s[1] * inv_rho;
     mom[2] = s[2] * inv_rho;
     mom[3] = s[3] * inv_rho;
@@ -239,13 +238,14 @@ __device__ __forceinline__ void interior_moments(const float *s, float *mom)
 }
 
 // Wet-node boundary moments (unscaled), boundaryConditions.cuh:99-533, from
-// the folds of the known populations (s[0] = rho_I, s[5,6,8] = the raw
-// c_a c_b sums whose quotients by rho_I are the reference's m_ab_I).
+// the folds of the known populations (s[0] = rho_I, inv_rho_I = 1 / rho_I,
+// s[5,6,8] = the raw c_a c_b sums whose quotients by rho_I are the reference's
+// m_ab_I).
 template <int Q>
-__device__ __forceinline__ void boundary_moments(const float *s, unsigned t, const Relax &rx, float *mom)
+__device__ __forceinline__ void boundary_moments(const float *s, float inv_rho_I, unsigned t, const Relax &rx,
+                                                 float *mom)
 {
     const float rho_I = s[0];
-    const float inv_rho_I = 1.0f / rho_I;
     const float omega = rx.omega;
     const float U = rx.u_lid;
 
@@ -487,10 +487,12 @@ __device__ __forceinline__ void scale_collide(float *m, const Relax &rx)
 template <int Q, int SCI = 1>
 __device__ __forceinline__ void node_update(const float *s, unsigned type, const Relax &rx, float *m)
 {
+    // one reciprocal for both kinds of node: a warp with a wall runs both
+    const float inv = 1.0f / s[0];
     if (type)
-        boundary_moments<Q>(s, type, rx, m);
+        boundary_moments<Q>(s, inv, type, rx, m);
     else
-        interior_moments(s, m);
+        interior_moments(s, inv, m);
     scale_collide<SCI>(m, rx);
 }
 
