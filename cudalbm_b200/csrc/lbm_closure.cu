@@ -587,7 +587,7 @@ lbm_status launch_infer(const float *src, size_t N, const MlpDevice &net, float 
     uint64_t timeout = 2000000000ull;
     MlpDevice net_arg = net;
     void *args[] = {&src, &N, &net_arg, &out, &err, &timeout};
-    LBM_CUDA_RETURN(cudaLaunchKernel(fn, dim3(grid), dim3(128), args, lbm::MlpSmem::LAUNCH_BYTES, stream));
+    LBM_CUDA_RETURN(lbm::launch_overlapped(fn, dim3(grid), dim3(128), args, lbm::MlpSmem::LAUNCH_BYTES, stream));
     return LBM_OK;
 }
 

@@ -1076,6 +1076,7 @@ __global__ void __launch_bounds__(TX *TY, MINB)
     f.row = lin & 127;
     f.group = grp;
     f.leader = (lin & 127) == 0;
+    f.issuer = (__shfl_sync(0xffffffffu, warp, 0) & 3) == 0;
     f.ph1 = f.ph2 = 0u;
     f.in_prev = f.in_cur = false;
     MonAcc acc;
