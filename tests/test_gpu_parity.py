@@ -90,6 +90,19 @@ def test_default_shape_equals_a_named_one(q, shape, storage):
     assert bits_equal(out["moments"], base["moments"])
 
 
+@pytest.mark.parametrize("q,tile,npb,storage,fo", [(19, 32, 4, "f32", ()), (27, 32, 1, "f16", ()), (27, 16, 1, "f32", ("k",)),
+                                                   (19, 32, 2, "f32", ()), (27, 8, 1, "f32", ("S", "momentsMean"))])
+@pytest.mark.parametrize("z_chunk", [1, 2, 3])
+def test_shortest_chunks(q, tile, npb, storage, fo, z_chunk):
+    """Items of one, two and three planes between their first plane (up-movers
+    only) and their last (down-movers only): the bits of 8-plane items."""
+    kw = dict(fo=fo, storage=storage, tile=(tile, 8, 2), pop_buffers=npb)
+    base = run_cavity(q, 40, 16, 24, 400.0, 0.05, 9, z_chunk=8, **kw)
+    out = run_cavity(q, 40, 16, 24, 400.0, 0.05, 9, z_chunk=z_chunk, **kw)
+    for k in base:
+        assert bits_equal(out[k], base[k]), k
+
+
 @pytest.mark.parametrize("q,tile,npb", [(19, 32, 1), (19, 32, 4), (27, 32, 1), (27, 16, 1), (27, 8, 1)])
 @pytest.mark.parametrize("mean_bits", [32, 64])
 def test_function_object_kernels_agree(q, tile, npb, mean_bits):
