@@ -272,6 +272,7 @@ void default_tiling(int64_t nx, int64_t ny, int64_t nz, int only_tx, bool narrow
     constexpr Tile kTiles[] = {{32, 1.1, 0.33, 0.55}, {16, 1.1, 0.6, 0.29}, {8, 1.1, 0.6, 0.21}};
     constexpr double kSms = 148.0;
     double best = 1e300;
+    zc = int((nz + 65534) / 65535);  // the grid's z limit, for meshes longer than any chunk below allows
     for (const Tile &t : kTiles) {
         if (only_tx ? t.tx != only_tx : (t.tx == 8 && !narrow) || (t.tx > 8 && nx <= t.tx / 2 && (narrow || t.tx > 16)))
             continue;
@@ -280,6 +281,8 @@ void default_tiling(int64_t nx, int64_t ny, int64_t nz, int only_tx, bool narrow
             if (c > nz)
                 continue;
             const lbm::ZChunks z = lbm::z_chunks(nz, c, tiles, t.tx * 8 / 32);
+            if (z.count > 65535)
+                continue;
             double us;
             if (z.zc2 != z.zc)
                 us = t.per_cta * double(tiles) * double(nz + 2 * z.count) / kSms + 0.5 * t.base * (c + 2);

@@ -1114,6 +1114,11 @@ lbm_status lbm_trainer_fit(lbm_trainer *t, const lbm_train_options *opt, lbm_mlp
     LBM_CUDA_RETURN(cudaSetDevice(t->device));
     const uint64_t B = uint64_t(opt->batch);
     const unsigned blocks = unsigned((B + kTrainCta - 1) / kTrainCta);
+    // the losses of the first and the last tenth are kept (one slot for the
+    // steps between) and read once at the end
+    const int window = std::max(1, std::min(opt->steps / 10, 100)), last = opt->steps - window;
+    auto loss_slot = [&](int step) { return size_t(step < window ? step : step >= last ? window + step - last : 2 * window); };
+    std::vector<double> losses(size_t(2 * window + 1));
     MlpParams *dp = nullptr;
     float *dm = nullptr, *dv = nullptr, *dpart = nullptr;
     double *dl = nullptr, *dlpart = nullptr;
@@ -1126,7 +1131,7 @@ lbm_status lbm_trainer_fit(lbm_trainer *t, const lbm_train_options *opt, lbm_mlp
         cudaFree(dlpart);
     };
     if (cudaMalloc(&dp, sizeof(MlpParams)) != cudaSuccess || cudaMalloc(&dm, kMlpWeights * 4) != cudaSuccess || cudaMalloc(&dv, kMlpWeights * 4) != cudaSuccess ||
-        cudaMalloc(&dl, size_t(opt->steps) * sizeof(double)) != cudaSuccess ||
+        cudaMalloc(&dl, losses.size() * sizeof(double)) != cudaSuccess ||
         cudaMalloc(&dpart, size_t(blocks) * kMlpWeights * 4) != cudaSuccess ||
         cudaMalloc(&dlpart, blocks * sizeof(double)) != cudaSuccess) {
         release();
@@ -1136,12 +1141,11 @@ lbm_status lbm_trainer_fit(lbm_trainer *t, const lbm_train_options *opt, lbm_mlp
     cudaMemset(dm, 0, kMlpWeights * 4);
     cudaMemset(dv, 0, kMlpWeights * 4);
     cudaFuncSetAttribute(grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(TrainSmem)));
-    const int window = std::max(1, std::min(opt->steps / 10, 100));
     cudaError_t e = cudaSuccess;
     for (int step = 0; step < opt->steps && e == cudaSuccess; step++) {
         uint64_t first = 0, seed = splitmix64(opt->seed + 0x51ED27ull * uint64_t(step + 1));
         int random = 1, ctas = int(blocks);
-        double *loss = dl + step;
+        double *loss = dl + loss_slot(step);
         float c1 = 1.0f / (1.0f - std::pow(0.9f, float(step + 1))), c2 = 1.0f / (1.0f - std::pow(0.999f, float(step + 1)));
         float lr = opt->lr, *w = reinterpret_cast<float *>(dp);
         uint64_t batch = B;
@@ -1153,8 +1157,6 @@ lbm_status lbm_trainer_fit(lbm_trainer *t, const lbm_train_options *opt, lbm_mlp
             e = lbm::launch_overlapped(reinterpret_cast<const void *>(&reduce_adam_kernel),
                                        dim3(kMlpWeights / kAdamCta + 1), dim3(kAdamCta), aa, 0, t->stream);
     }
-    // every step's loss, read once at the end
-    std::vector<double> losses(size_t(opt->steps));
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(losses.data(), dl, losses.size() * sizeof(double), cudaMemcpyDeviceToHost, t->stream);
     const cudaError_t es = cudaStreamSynchronize(t->stream);
@@ -1164,7 +1166,7 @@ lbm_status lbm_trainer_fit(lbm_trainer *t, const lbm_train_options *opt, lbm_mlp
     int acc_n = 0;
     for (int step = 0; step < opt->steps; step++)
         if (step < window || step >= opt->steps - window) {
-            acc += losses[size_t(step)] / double(B);
+            acc += losses[loss_slot(step)] / double(B);
             if (++acc_n == window) {
                 if (first_loss < 0.0)
                     first_loss = acc / window;

@@ -128,6 +128,8 @@ __global__ void __launch_bounds__(kOrderedThreads) ordered_sum_kernel(const floa
         size_t z = row / size_t(ny);
         for (int j = id; j < kOrderedChunk && g < g1; j += kFetchers, g += kFetchers) {
             dst[j] = __ldg(f + (tiled ? tiled_address(x, y, z, nx >> 3, ny >> 3) : g));
+            if (!tiled)
+                continue;
             x += kFetchers;
             while (x >= nx) {
                 x -= nx;

@@ -193,7 +193,10 @@ inline ZChunks z_chunks(int64_t nz, int zc, int64_t tiles, int warps)
     if (zc < 16 || tiles * uniform * warps < 2 * kSms * kResidentWarps || nz < 2 * zc)
         return {zc, uniform, zc, uniform};
     const int nbig = int((nz - (3 * zc + 3) / 4) / zc), zc2 = (zc + 3) / 4;
-    return {zc, nbig, zc2, nbig + int((nz - int64_t(nbig) * zc + zc2 - 1) / zc2)};
+    const int count = nbig + int((nz - int64_t(nbig) * zc + zc2 - 1) / zc2);
+    if (count > 65535)  // the grid's z limit
+        return {zc, uniform, zc, uniform};
+    return {zc, nbig, zc2, count};
 }
 
 template <int TX, int TY, typename ST = float>
