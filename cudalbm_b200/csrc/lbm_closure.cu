@@ -648,6 +648,25 @@ struct lbm_trainer {
 
 namespace lbm {
 
+// Lets a kernel take `smem` bytes of shared memory, once per kernel and device
+// (the call is far slower than a launch).
+static lbm_status allow_smem(const void *fn, int device, size_t smem)
+{
+    struct Known {
+        const void *fn;
+        int device;
+    };
+    static std::mutex mu;
+    static std::vector<Known> known;
+    std::lock_guard<std::mutex> lock(mu);
+    for (const Known &k : known)
+        if (k.fn == fn && k.device == device)
+            return LBM_OK;
+    LBM_CUDA_RETURN(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    known.push_back({fn, device});
+    return LBM_OK;
+}
+
 // One step of a handle with the closure: dtau from the current moments on
 // the tensor cores, then the closure step kernel.
 lbm_status closure_step(lbm_handle *h)
@@ -658,22 +677,9 @@ lbm_status closure_step(lbm_handle *h)
         pick_closure_fused(h->Q, h->launcher.tx, h->launcher.ty, h->launcher.stages, h->launcher.pop_buffers, ffn,
                            fsmem)) {
         // the network inside the step kernel: no dtau array, one launch
-        struct Known {
-            const void *fn;
-            int device;
-        };
-        static std::mutex mu;
-        static std::vector<Known> known;
-        {
-            std::lock_guard<std::mutex> lock(mu);
-            bool seen = false;
-            for (const Known &k : known)
-                seen |= (k.fn == ffn && k.device == h->cfg.device);
-            if (!seen) {
-                LBM_CUDA_RETURN(cudaFuncSetAttribute(ffn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(fsmem)));
-                known.push_back({ffn, h->cfg.device});
-            }
-        }
+        lbm_status as = allow_smem(ffn, h->cfg.device, fsmem);
+        if (as != LBM_OK)
+            return as;
         StepParams<float, float> p{};
         const int nxt = h->cur ^ 1;
         p.out = static_cast<float *>(h->m[nxt]);
@@ -716,6 +722,9 @@ lbm_status closure_step(lbm_handle *h)
     size_t smem = 0;
     if (!pick_closure(h->Q, h->launcher.tx, h->launcher.ty, h->launcher.stages, h->launcher.pop_buffers, fn, smem))
         return fail(LBM_ERR_STATE, "closure: the handle's kernel shape has no closure variant");
+    lbm_status as = allow_smem(fn, h->cfg.device, smem);  // the autotuner moves between shapes
+    if (as != LBM_OK)
+        return as;
     StepParams<float, float> p{};
     const int nxt = h->cur ^ 1;
     p.out = static_cast<float *>(h->m[nxt]);

@@ -240,6 +240,22 @@ def test_fused_network_equals_separate_kernels(samples, q, nx):
         assert np.array_equal(bits(da2), bits(db2)) and not np.array_equal(bits(da2), bits(da))
 
 
+@pytest.mark.parametrize("tile", [8, 16])
+def test_autotune_moves_between_closure_shapes(samples, tile):
+    """The autotuner may leave the shape the closure was set with for one
+    that needs more shared memory; the steps keep their bits."""
+    _, feats, targ, _, _ = samples
+    net = random_net(feats, targ, seed=5, scale=0.5)
+    with Cavity(19, 40, 16, 24, 300.0, 0.05, tile=(tile, 8, 2)) as a, Cavity(19, 40, 16, 24, 300.0, 0.05) as b:
+        for c in (a, b):
+            c.init_regions()
+            c.set_closure(net)
+        a.autotune(4)
+        a.step(5)
+        b.step(5)
+        assert np.array_equal(bits(a.read()), bits(b.read()))
+
+
 def test_autotune_picks_the_closure_evaluation_and_keeps_the_state(samples):
     """With a closure set, the autotuner times the closure kernel shapes and
     both evaluations of the network (inside the step kernel, or a separate
