@@ -260,9 +260,9 @@ bool pick_launcher(int Q, int tx, int ty, int stages, int npb, int storage, unsi
 // chunk of draining.  Tiles with more than half of their lanes outside the
 // mesh are left out.  Over 38 meshes from 32x16x24 to 192^3 the choice is
 // within 15% of the fastest (tile, z-chunk), 3% on average.  D3Q19, us per
-// step, the former rule (widest tile that divides nx, chunks of 9 or more) ->
-// this one: 32x16x24 16.4 -> 4.1, 8x64x64 24.1 -> 5.2, 64^3 20.3 -> 9.5,
-// 88x96x104 30.0 -> 24.9, 296x264x248 690 -> 317.
+// step, the former rule (widest tile that divides nx, chunks of 9 or more,
+// former kernels) -> this one: 32x16x24 20.6 -> 3.6, 8x64x64 29.1 -> 4.5,
+// 64^3 24.0 -> 8.8, 88x96x104 33.2 -> 23.2, 296x264x248 667 -> 304.
 void default_tiling(int64_t nx, int64_t ny, int64_t nz, int only_tx, bool narrow, int &tx, int &zc)
 {
     struct Tile {

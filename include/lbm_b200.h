@@ -77,7 +77,7 @@ typedef struct lbm_config {
     uint32_t function_objects;/* LBM_FO_* mask */
     int32_t mean_bits;        /* 32: float running means as the reference; 64: double accumulators */
     int64_t start_step;       /* absolute step index of the initial state (restart: latestTime) */
-    /* kernel tiling; 0 = autotuned choice for this size class */
+    /* kernel tiling; 0 = chosen for the mesh by a measured cost (lbm_autotune times the candidates) */
     int32_t tile_x, tile_y, z_chunk, stages;
     int32_t pop_buffers;      /* shared-memory population planes: 1 (two barriers per plane, 3 CTAs/SM),
                                  2 (one barrier per plane), 4 (one plane, 4 CTAs/SM; D3Q19 shapes) */
@@ -209,7 +209,7 @@ lbm_status lbm_get_info(lbm_handle *h, lbm_info *info);
 /* Kernel variant chosen by lbm_autotune. */
 typedef struct lbm_tuning {
     int32_t tile_x, tile_y;   /* x-y tile of one CTA */
-    int32_t z_chunk;          /* z-planes per CTA */
+    int32_t z_chunk;          /* z-planes per CTA (a large grid ends in quarter chunks) */
     int32_t stages;           /* TMA pipeline depth (moment planes in flight) */
     int32_t pop_buffers;      /* 1: one population plane, 3 CTAs/SM; 2: two planes; 4: one plane, 4 CTAs/SM */
     double ms_per_step;       /* measured device time per step of the chosen variant */
