@@ -1040,14 +1040,20 @@ lbm_status lbm_trainer_gradient(lbm_trainer *t, const lbm_mlp *net, uint64_t fir
         release();
         return fail(LBM_ERR_NOMEM, "lbm_trainer_gradient: no device memory");
     }
-    cudaMemcpy(dp, net, sizeof(MlpParams), cudaMemcpyHostToDevice);
-    cudaFuncSetAttribute(grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(TrainSmem)));
-    grad_kernel<<<ctas, kTrainThreads, sizeof(TrainSmem), t->stream>>>(t->feat, t->targ, n, first, count, 0, 0, dp,
-                                                                   dpart, dlpart);
-    reduce_partials_kernel<<<(kMlpWeights + 255) / 256, 256, 0, t->stream>>>(dpart, dlpart, int(ctas), dg, dl);
-    cudaError_t e = cudaGetLastError();
+    // uploads go on the trainer's stream: it does not wait for the legacy
+    // default stream, on which a plain cudaMemcpy or cudaMemset runs
+    cudaError_t e = cudaMemcpyAsync(dp, net, sizeof(MlpParams), cudaMemcpyHostToDevice, t->stream);
     if (e == cudaSuccess)
-        e = cudaStreamSynchronize(t->stream);
+        e = cudaFuncSetAttribute(grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(TrainSmem)));
+    if (e == cudaSuccess) {
+        grad_kernel<<<ctas, kTrainThreads, sizeof(TrainSmem), t->stream>>>(t->feat, t->targ, n, first, count, 0, 0, dp,
+                                                                       dpart, dlpart);
+        reduce_partials_kernel<<<(kMlpWeights + 255) / 256, 256, 0, t->stream>>>(dpart, dlpart, int(ctas), dg, dl);
+        e = cudaGetLastError();
+    }
+    const cudaError_t es = cudaStreamSynchronize(t->stream);
+    if (e == cudaSuccess)
+        e = es;
     if (e == cudaSuccess) {
         std::memset(grad, 0, sizeof(*grad));
         e = cudaMemcpy(grad, dg, kMlpWeights * sizeof(float), cudaMemcpyDeviceToHost);
@@ -1146,11 +1152,13 @@ lbm_status lbm_trainer_fit(lbm_trainer *t, const lbm_train_options *opt, lbm_mlp
         release();
         return fail(LBM_ERR_NOMEM, "lbm_trainer_fit: no device memory");
     }
-    cudaMemcpy(dp, &P, sizeof(P), cudaMemcpyHostToDevice);
-    cudaMemset(dm, 0, kMlpWeights * 4);
-    cudaMemset(dv, 0, kMlpWeights * 4);
-    cudaFuncSetAttribute(grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(TrainSmem)));
-    cudaError_t e = cudaSuccess;
+    // on the trainer's stream, as the kernels that read them (see lbm_trainer_gradient)
+    cudaError_t e = cudaMemcpyAsync(dp, &P, sizeof(P), cudaMemcpyHostToDevice, t->stream);
+    for (float *moment : {dm, dv})
+        if (e == cudaSuccess)
+            e = cudaMemsetAsync(moment, 0, kMlpWeights * 4, t->stream);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(TrainSmem)));
     for (int step = 0; step < opt->steps && e == cudaSuccess; step++) {
         uint64_t first = 0, seed = splitmix64(opt->seed + 0x51ED27ull * uint64_t(step + 1));
         int random = 1, ctas = int(blocks);

@@ -176,6 +176,32 @@ def test_training_lowers_the_loss(samples):
     assert np.all(np.isfinite(np.array(net.w2)))
 
 
+def test_training_does_not_depend_on_work_on_the_default_stream(samples):
+    """Weights, Adam's moments and their uploads are ordered by the trainer's
+    stream: with the legacy default stream busy for a while, a gradient and a
+    training run give the bits they give on a quiet GPU."""
+    import torch
+
+    tr, feats, targ, _, _ = samples
+    net = random_net(feats, targ, seed=6)
+
+    def results(busy):
+        out = []
+        for call in (lambda: tr.gradient(net, 0, 300), lambda: tr.fit(steps=12, batch=512, seed=4)):
+            if busy:
+                torch.cuda._sleep(int(1e8))  # about 50 ms, one block
+            n, rep = call()
+            out += [np.array(getattr(n, w)) for w in ("w1", "b1", "w2", "b2", "w3", "b3")]
+            out.append(np.array(list(rep.values()) if isinstance(rep, dict) else rep))
+            torch.cuda.synchronize()
+        return out
+
+    quiet, busy = results(False), results(True)
+    assert all(np.all(np.isfinite(a)) for a in quiet)
+    for a, b in zip(quiet, busy):
+        assert np.array_equal(a, b)
+
+
 def test_samples_and_training_are_reproducible():
     tr1, _, _ = make_samples(q=19, n=32, steps=20, seed=5, snapshots=1)
     tr2, _, _ = make_samples(q=19, n=32, steps=20, seed=5, snapshots=1)
