@@ -198,10 +198,14 @@ lbm_status build_tables(lbm_batch *b)
     if (per_sm < 1)
         return fail(LBM_ERR_CUDA, "batch: the kernel shape does not fit on one SM");
     b->grid = b->persistent ? int(std::min<int64_t>(int64_t(per_sm) * sms, items)) : int(items);
-    // the previous launches read the tables: order the uploads after them
+    // The uploads follow the launches that read the tables and precede the
+    // next ones: on the batch's stream, which does not wait for the legacy
+    // default stream (the host arrays are staged before each call returns).
     LBM_CUDA_RETURN(cudaStreamSynchronize(b->stream));
-    LBM_CUDA_RETURN(cudaMemcpy(b->d_mesh, mesh.data(), sizeof(lbm::BatchMesh) * n, cudaMemcpyHostToDevice));
-    LBM_CUDA_RETURN(cudaMemcpy(b->d_tmap, tmap.data(), sizeof(CUtensorMap) * 2 * n, cudaMemcpyHostToDevice));
+    LBM_CUDA_RETURN(cudaMemcpyAsync(b->d_mesh, mesh.data(), sizeof(lbm::BatchMesh) * n, cudaMemcpyHostToDevice,
+                                    b->stream));
+    LBM_CUDA_RETURN(cudaMemcpyAsync(b->d_tmap, tmap.data(), sizeof(CUtensorMap) * 2 * n, cudaMemcpyHostToDevice,
+                                    b->stream));
     b->h_mesh = mesh;
     b->tables_valid = true;
     drop_graph(b);
@@ -222,8 +226,8 @@ lbm_status refresh(lbm_batch *b)
     for (size_t i = 0; i < b->cav.size(); i++)
         b->h_mesh[b->row_of[i]].cur = b->cav[i]->cur;
     LBM_CUDA_RETURN(cudaStreamSynchronize(b->stream));
-    LBM_CUDA_RETURN(cudaMemcpy(b->d_mesh, b->h_mesh.data(), sizeof(lbm::BatchMesh) * b->cav.size(),
-                               cudaMemcpyHostToDevice));
+    LBM_CUDA_RETURN(cudaMemcpyAsync(b->d_mesh, b->h_mesh.data(), sizeof(lbm::BatchMesh) * b->cav.size(),
+                                    cudaMemcpyHostToDevice, b->stream));
     return LBM_OK;
 }
 
@@ -357,7 +361,8 @@ lbm_status lbm_batch_create(const lbm_config *cfgs, int32_t n, lbm_batch **out)
         cudaMalloc(&b->d_ctr, 2 * sizeof(unsigned)) != cudaSuccess || cudaMalloc(&b->d_err, sizeof(lbm::StepFault)) != cudaSuccess)
         return cleanup(fail(LBM_ERR_NOMEM, "lbm_batch_create: cannot allocate the batch tables"));
     b->table_bytes = sizeof(lbm::BatchMesh) * n + sizeof(CUtensorMap) * 2 * size_t(n) + 2 * sizeof(unsigned) + sizeof(lbm::StepFault);
-    if (cudaMemset(b->d_ctr, 0, 2 * sizeof(unsigned)) != cudaSuccess || cudaMemset(b->d_err, 0, sizeof(lbm::StepFault)) != cudaSuccess)
+    if (cudaMemsetAsync(b->d_ctr, 0, 2 * sizeof(unsigned), b->stream) != cudaSuccess ||
+        cudaMemsetAsync(b->d_err, 0, sizeof(lbm::StepFault), b->stream) != cudaSuccess)
         return cleanup(fail(LBM_ERR_CUDA, "lbm_batch_create: cannot clear the batch counters"));
     int tx;
     default_shape(b, tx);

@@ -51,6 +51,31 @@ def test_batch_is_bitwise_equal_to_single_cavities(specs):
             assert np.array_equal(bits(b[i].read()), bits(alone(sp, 9))), i
 
 
+def test_batch_does_not_depend_on_work_on_the_default_stream():
+    """Work counters, mesh table and TMA descriptors are ordered by the
+    batch's stream: a batch created, reshaped and stepped an odd number of
+    steps while the legacy default stream is busy gives the same bits."""
+    import torch
+
+    ref = [alone(sp, 8) for sp in SPECS19]
+    busy = lambda: torch.cuda._sleep(int(1e8))  # noqa: E731  (about 50 ms, one block)
+    busy()
+    with Batch(SPECS19) as b:
+        b.init_regions()
+        busy()
+        b.step(3)
+        busy()
+        b.step(2)  # tables refreshed: the buffers changed places
+        b.synchronize()
+        busy()
+        b.configure(16)
+        b.step(3)
+        b.synchronize()
+        for i in range(len(b)):
+            assert np.array_equal(bits(b[i].read()), bits(ref[i])), i
+    torch.cuda.synchronize()
+
+
 def test_batch_shapes_and_chunks_do_not_change_results():
     ref = [alone(sp, 6) for sp in SPECS19]
     with Batch(SPECS19) as b:
