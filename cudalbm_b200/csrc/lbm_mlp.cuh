@@ -31,6 +31,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <cstddef>
 #include <cstdint>
 
 #include "lbm_ptx.cuh"
@@ -51,8 +52,10 @@ struct MlpParams {
 constexpr int kMlpWeights = kMlpHidden * kMlpIn + kMlpHidden + kMlpHidden * kMlpHidden + kMlpHidden + kMlpHidden + 1;
 
 // Device copy for the tensor-core path: FP16 weights already in the operand
-// layout (umma_index), FP32 vectors.
-struct MlpDevice {
+// layout (umma_index), FP32 vectors.  Aligned, so that a kernel parameter of
+// this type starts on 16 bytes whatever stands in front of it: the biases are
+// read two at a time (biased_f16x2).
+struct alignas(16) MlpDevice {
     __half w1[kMlpHidden * kMlpIn];      // [32 out][16 in]
     __half w2[kMlpHidden * kMlpHidden];  // [32 out][32 in]
     float b1[kMlpHidden], b2[kMlpHidden], w3[kMlpHidden], b3;
@@ -60,6 +63,8 @@ struct MlpDevice {
     float out_scale, dtau_lo, dtau_hi;
     float r_ii, r_ij;  // 1 / (2 * 4.5 * tau0), 1 / (2 * 9 * tau0) for the strain-rate features
 };
+static_assert(alignof(MlpDevice) % 8 == 0 && offsetof(MlpDevice, b1) % 8 == 0 && offsetof(MlpDevice, b2) % 8 == 0,
+              "biased_f16x2 reads pairs of biases as 8 bytes");
 
 // Element (row, k) of a rows x K FP16 operand in the K-major, no-swizzle
 // canonical layout: core matrices of 8 rows x 8 elements (16 B per row,
@@ -87,10 +92,11 @@ __device__ __forceinline__ uint32_t pack_f16x2_sat(float lo, float hi)
 }
 
 // Two accumulators plus their biases (one packed FP32 addition, each half
-// rounded like the scalar one), as FP16x2.  The accumulators come out of
-// tensor memory in consecutive registers, so the pair costs no moves; with the
-// issue confined to one warp and the range check chained, mlp_infer_kernel
-// went from 811 to 688 instructions per node and 74.8 to 69.8 us (128^3).
+// rounded like the scalar one), as FP16x2; b is 8-byte aligned.  The
+// accumulators come out of tensor memory in consecutive registers, so the pair
+// costs no moves; with the issue confined to one warp and the range check
+// chained, mlp_infer_kernel went from 811 to 688 instructions per node and
+// 74.8 to 69.8 us (128^3).
 __device__ __forceinline__ uint32_t biased_f16x2(const float *z, const float *b)
 {
     uint64_t zz, r;
@@ -492,7 +498,6 @@ __global__ void __launch_bounds__(128, kMlpCtasPerSm) mlp_infer_kernel(const flo
     const bool leader = tid == 0;
 
     // weights (already in operand layout) into shared memory, 4 B at a time
-    // (the parameter block guarantees 4-byte alignment)
     {
         const uint32_t *g = reinterpret_cast<const uint32_t *>(net.w1);
         uint32_t *d = reinterpret_cast<uint32_t *>(sm + MlpSmem::W1);
