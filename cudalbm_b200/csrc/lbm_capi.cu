@@ -396,18 +396,25 @@ lbm_status ensure_scratch(lbm_handle *h, size_t bytes)
     return LBM_OK;
 }
 
-// Monitor slots for n steps.
+// Steps of lbm_step_monitored that share a memset and a copy; a handle has
+// slots for as many from its creation on (96 KB), so that no monitored call
+// allocates.
+constexpr uint64_t kMonBlock = 4096;
+
+// Monitor slots for n steps (more than kMonBlock: a long lbm_run_streamed).
+// The old slots stay until the new ones are there.
 lbm_status ensure_mon_steps(lbm_handle *h, uint64_t n)
 {
     if (h->mon_steps_cap >= n)
         return LBM_OK;
+    lbm::MonitorSlot *slots = nullptr;
+    LBM_CUDA(cudaMalloc(&slots, n * sizeof(lbm::MonitorSlot)));
     if (h->mon_steps) {
+        cudaStreamSynchronize(h->stream);  // monitored steps still queued write the old ones
         cudaFree(h->mon_steps);
         h->device_bytes -= h->mon_steps_cap * sizeof(lbm::MonitorSlot);
-        h->mon_steps = nullptr;
-        h->mon_steps_cap = 0;
     }
-    LBM_CUDA(cudaMalloc(&h->mon_steps, n * sizeof(lbm::MonitorSlot)));
+    h->mon_steps = slots;
     h->mon_steps_cap = n;
     h->device_bytes += n * sizeof(lbm::MonitorSlot);
     return LBM_OK;
@@ -861,6 +868,7 @@ lbm_status lbm_create(const lbm_config *cfg, lbm_handle **out)
         if ((s = dev_alloc(h, reinterpret_cast<char **>(&h->momentsMean), 10 * h->N * msz)) != LBM_OK) return cleanup_fail(s);
     if ((s = dev_alloc(h, &h->err, 1)) != LBM_OK) return cleanup_fail(s);
     if ((s = dev_alloc(h, &h->red, 4)) != LBM_OK) return cleanup_fail(s);
+    if ((s = ensure_mon_steps(h, kMonBlock)) != LBM_OK) return cleanup_fail(s);
     for (int b = 0; b < 2; b++) {
         cudaMemsetAsync(h->m[b], 0, 10 * h->N * h->esz, h->stream);
     }
@@ -1128,12 +1136,9 @@ lbm_status lbm_step_monitored(lbm_handle *h, uint64_t n, lbm_monitor *out)
         return LBM_OK;
     // a slot per step, zeroed and copied to the host in blocks: with a memset
     // and a copy around every step the steps cannot overlap
-    constexpr uint64_t kMonBlock = 4096;
-    lbm_status s = ensure_mon_steps(h, std::min(n, kMonBlock));
-    if (s != LBM_OK)
-        return s;
     LBM_CUDA(cudaEventRecord(h->ev0, h->stream));
     const bool md = means_f64(h);
+    lbm_status s;
     for (uint64_t b = 0; b < n; b += kMonBlock) {
         const uint64_t cnt = std::min(n - b, kMonBlock);
         LBM_CUDA(cudaMemsetAsync(h->mon_steps, 0, cnt * sizeof(lbm::MonitorSlot), h->stream));

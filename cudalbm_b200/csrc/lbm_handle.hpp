@@ -42,7 +42,7 @@ struct lbm_handle {
     cudaEvent_t xe_converted[2] = {nullptr, nullptr};
     // lbm_run_streamed: uploads go on xstream, downloads on dstream
     cudaStream_t dstream = nullptr;
-    lbm::MonitorSlot *mon_steps = nullptr;  // a slot per monitored step of a call (or of a block of its steps)
+    lbm::MonitorSlot *mon_steps = nullptr;  // a slot per monitored step of a block or of a streamed job
     size_t mon_steps_cap = 0;
     float tau = 0, omega = 0, t_omega = 0, omega_d2 = 0;
     int64_t t = 0;
