@@ -23,6 +23,7 @@
 #include "casefile.hpp"
 #include "lbm_b200.h"
 #include "lbm_handle.hpp"
+#include "lbm_monitor.hpp"
 #include "lbm_mlp.cuh"
 #include "lbm_step.cuh"
 #include "lbmbin.hpp"
@@ -1138,16 +1139,25 @@ lbm_status lbm_step_monitored(lbm_handle *h, uint64_t n, lbm_monitor *out)
     // and a copy around every step the steps cannot overlap
     LBM_CUDA(cudaEventRecord(h->ev0, h->stream));
     const bool md = means_f64(h);
-    lbm_status s;
-    for (uint64_t b = 0; b < n; b += kMonBlock) {
-        const uint64_t cnt = std::min(n - b, kMonBlock);
-        LBM_CUDA(cudaMemsetAsync(h->mon_steps, 0, cnt * sizeof(lbm::MonitorSlot), h->stream));
-        for (uint64_t i = 0; i < cnt; i++)
-            if ((s = md ? launch_step<double>(h, h->mon_steps + i) : launch_step<float>(h, h->mon_steps + i)) != LBM_OK)
-                return s;
-        LBM_CUDA(cudaMemcpyAsync(out + b, h->mon_steps, cnt * sizeof(lbm::MonitorSlot), cudaMemcpyDeviceToHost,
-                                 h->stream));
-    }
+    const lbm_status s = lbm::monitored_blocks(
+        n, kMonBlock,
+        [&](uint64_t count) -> lbm_status {
+            LBM_CUDA(cudaMemsetAsync(h->mon_steps, 0, count * sizeof(lbm::MonitorSlot), h->stream));
+            return LBM_OK;
+        },
+        [&](uint64_t slot) {
+            return md ? launch_step<double>(h, h->mon_steps + slot) : launch_step<float>(h, h->mon_steps + slot);
+        },
+        [&](uint64_t first, uint64_t count, bool failed) -> lbm_status {
+            const cudaError_t e = cudaMemcpyAsync(out + first, h->mon_steps, count * sizeof(lbm::MonitorSlot),
+                                                  cudaMemcpyDeviceToHost, h->stream);
+            if (failed)  // the message stays the failed launch's
+                return LBM_OK;
+            LBM_CUDA(e);
+            return LBM_OK;
+        });
+    if (s != LBM_OK)
+        return s;
     LBM_CUDA(cudaEventRecord(h->ev1, h->stream));
     h->timed = true;
     return LBM_OK;

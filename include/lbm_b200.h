@@ -149,7 +149,9 @@ typedef struct lbm_monitor {
 /* lbm_step with a per-step result: step i writes its sums to out[i] (n
  * entries); an asynchronous device-to-host copy follows the steps (every 4096).
  * With page-locked `out` (lbm_host_alloc) nothing waits for the host; the
- * values are valid after lbm_synchronize.  Replaces: the reference's per-step
+ * values are valid after lbm_synchronize.  If a step cannot be launched the
+ * call returns its error, and the results of the steps before it still arrive.
+ * Replaces: the reference's per-step
  * info print (momentBasedD3Q19.cu:107-110) and fieldCalculate containsNaN
  * (applications/fieldCalculate/fieldCalculate.cuh:74-110), at no extra pass. */
 lbm_status lbm_step_monitored(lbm_handle *h, uint64_t n, lbm_monitor *out);
