@@ -608,11 +608,14 @@ lbm_status launch_step(lbm_handle *h, lbm::MonitorSlot *mon = nullptr)
     return LBM_OK;
 }
 
-// Step t of the planes [z_lo, z_hi) only, reading buffer `in` and writing the
-// other one (lbm_run_streamed); mon: the step's monitor slot or null.  The
-// handle's step counter and buffer index are left alone.
+// Step t of the planes [z_lo, z_hi) only, cut into the chunks zch, reading
+// buffer `in` and writing the other one (lbm_run_streamed); mon: the step's
+// monitor slot or null.  The handle's step counter and buffer index are left
+// alone.  Steps of the whole mesh are launched as launch_step does, since the
+// handle's z-chunk was chosen (or timed) for such launches.
 template <typename MeanT>
-lbm_status launch_slab(lbm_handle *h, int in, int64_t t, int z_lo, int z_hi, int zc, lbm::MonitorSlot *mon)
+lbm_status launch_slab(lbm_handle *h, int in, int64_t t, int z_lo, int z_hi, const lbm::ZChunks &zch,
+                       lbm::MonitorSlot *mon)
 {
     StepParams<MeanT> p{};
     p.out = static_cast<float *>(h->m[in ^ 1]);
@@ -620,8 +623,9 @@ lbm_status launch_slab(lbm_handle *h, int in, int64_t t, int z_lo, int z_hi, int
     p.nx = int(h->cfg.nx);
     p.ny = int(h->cfg.ny);
     p.nz = int(h->cfg.nz);
-    p.zc = p.zc2 = zc;
-    p.nbig = 0;
+    p.zc = zch.zc;
+    p.nbig = zch.nbig;
+    p.zc2 = zch.zc2;
     p.z_lo = z_lo;
     p.z_hi = z_hi;
     p.rx = lbm::Relax{h->omega, h->t_omega, h->omega_d2, h->tau, h->cfg.u_inf};
@@ -642,10 +646,13 @@ lbm_status launch_slab(lbm_handle *h, int in, int64_t t, int z_lo, int z_hi, int
     p.timeout_ns = 2000000000ull;
     const dim3 block(h->launcher.tx, h->launcher.ty);
     const dim3 grid(unsigned((h->cfg.nx + h->launcher.tx - 1) / h->launcher.tx),
-                    unsigned((h->cfg.ny + h->launcher.ty - 1) / h->launcher.ty), unsigned((z_hi - z_lo + zc - 1) / zc));
+                    unsigned((h->cfg.ny + h->launcher.ty - 1) / h->launcher.ty), unsigned(zch.count));
     void *args[] = {&h->tmap[in], &p};
-    LBM_CUDA(cudaLaunchKernel(mon ? h->launcher.fn_mon : h->launcher.fn, grid, block, args, h->launcher.smem,
-                              h->stream));
+    const void *fn = mon ? h->launcher.fn_mon : h->launcher.fn;
+    if (z_lo == 0 && z_hi == p.nz)
+        LBM_CUDA(lbm::launch_overlapped(fn, grid, block, args, h->launcher.smem, h->stream));
+    else
+        LBM_CUDA(cudaLaunchKernel(fn, grid, block, args, h->launcher.smem, h->stream));
     h->launches += 1;
     return LBM_OK;
 }
@@ -1261,11 +1268,11 @@ lbm_status lbm_run_streamed(lbm_handle *h, const float *moments, uint64_t n, voi
         return LBM_OK;
     };
     const bool md = means_f64(h);
-    auto step_range = [&](uint64_t s, int64_t lo, int64_t hi, int zcl) -> lbm_status {
+    auto step_range = [&](uint64_t s, int64_t lo, int64_t hi, const lbm::ZChunks &zch) -> lbm_status {
         const int in = int((uint64_t(in0) + s) & 1u);
         lbm::MonitorSlot *slot = mon ? h->mon_steps + s : nullptr;
-        return md ? launch_slab<double>(h, in, h->t + int64_t(s), int(lo), int(hi), zcl, slot)
-                  : launch_slab<float>(h, in, h->t + int64_t(s), int(lo), int(hi), zcl, slot);
+        return md ? launch_slab<double>(h, in, h->t + int64_t(s), int(lo), int(hi), zch, slot)
+                  : launch_slab<float>(h, in, h->t + int64_t(s), int(lo), int(hi), zch, slot);
     };
     std::vector<cudaEvent_t> up(size_t(U), nullptr);
     int waited = -1;  // upload chunks the compute stream has waited for
@@ -1291,7 +1298,8 @@ lbm_status lbm_run_streamed(lbm_handle *h, const float *moments, uint64_t n, voi
                 const int64_t hi = std::min<int64_t>(nz, bnd(j + 1) - int64_t(s));
                 if (lo >= hi)
                     continue;
-                lbm_status ls = step_range(s0 + s, lo, hi, zc);
+                const int count = int((hi - lo + zc - 1) / zc);
+                lbm_status ls = step_range(s0 + s, lo, hi, {zc, count, zc, count});
                 if (ls != LBM_OK)
                     return ls;
             }
@@ -1376,7 +1384,7 @@ lbm_status lbm_run_streamed(lbm_handle *h, const float *moments, uint64_t n, voi
         } else {
             ps = skewed(0, kSkew, true, false);
             for (uint64_t s = kSkew; ps == LBM_OK && s < n - kSkew; s++)
-                ps = step_range(s, 0, nz, h->zc);
+                ps = step_range(s, 0, nz, lbm::handle_chunks(h));
             if (ps == LBM_OK)
                 ps = skewed(n - kSkew, kSkew, false, true);
         }
