@@ -1791,12 +1791,19 @@ lbm_status lbm_autotune(lbm_handle *h, int32_t trial_steps, lbm_tuning *out)
         // (such a chunk re-reads two planes for every 2-4 it updates)
         const int64_t tiles = ((h->cfg.nx + v.tx - 1) / v.tx) * ((h->cfg.ny + v.ty - 1) / v.ty);
         const bool small = tiles * ((h->cfg.nz + 7) / 8) < 4 * 148 * 3;
-        // Candidates: a ladder of lengths, and, where the grid's end is not
-        // tapered (z_chunks), those whose grid is close to a whole number of
-        // waves of resident CTAs (k waves for k = 1..12): the last wave of a
-        // grid 9.2 waves long runs the GPU at a fifth of its CTA slots.
+        // Candidates: powers of two; where the grid's end is tapered
+        // (z_chunks), lengths between them, since any such chunk may be the
+        // best by a few percent; where it is not, those whose grid is close
+        // to a whole number of waves of resident CTAs (k waves for k = 1..12):
+        // the last wave of a grid 9.2 waves long runs the GPU at a fifth of
+        // its CTA slots.  Lengths between the powers of two on every grid made
+        // the call 1.5 times as long (78 lattices, meshes and field sets; 1.9
+        // times on the small ones) for steps that were no faster (1.0005).
         // Chunks need not divide nz (the last is shorter).
-        std::vector<int> zcs = {1, 2, 3, 4, 6, 8, 11, 16, 20, 26, 32, 37, 43, 52, 64};
+        std::vector<int> zcs = {2, 4, 8, 16, 32, 64};
+        for (int zc : {20, 26, 37, 43, 52})
+            if (const lbm::ZChunks z = lbm::z_chunks(h->cfg.nz, zc, tiles, v.tx * v.ty / 32); z.zc2 != z.zc)
+                zcs.push_back(zc);
         {
             Launcher l;
             int per_sm = 0;

@@ -40,3 +40,13 @@ def test_streamed_middle_steps(q, nx, storage, fo):
         b.synchronize()
         for s, out in outs.items():
             assert same_bits(out, b.read(s)), s
+
+
+@pytest.mark.parametrize("shape,most", [((64, 64, 64), 54), ((72, 40, 40), 42), ((8, 64, 64), 7)])
+def test_autotune_tries_few_chunks_where_none_tapers(shape, most):
+    """The lengths between the powers of two are timed on tapered grids only:
+    on a small mesh a call takes no longer than powers of two and whole waves."""
+    assert not tapers(*shape, 8, 16) and not tapers(*shape, 32, 16)
+    with Cavity(19, *shape, 400.0, 0.05) as c:
+        c.init_regions()
+        assert 0 < c.autotune()["candidates"] <= most
