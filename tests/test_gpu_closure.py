@@ -337,3 +337,90 @@ def test_window_targets():
     common = min(len(t0), len(t4))
     assert not np.array_equal(t4[:common], t0[:common])
     assert np.std(t4) < np.std(t0)  # the window averages out transition noise
+
+
+def splitmix64(x):
+    m = (1 << 64) - 1
+    x = (x + 0x9E3779B97F4A7C15) & m
+    x = ((x ^ (x >> 30)) * 0xBF58476D1CE4E5B9) & m
+    x = ((x ^ (x >> 27)) * 0x94D049BB133111EB) & m
+    return x ^ (x >> 31)
+
+
+def batch_loss(net, feats, targ, seed, step, batch):
+    """FP64 loss of `net` on the samples that training step `step` draws."""
+    key = splitmix64(seed + 0x51ED27 * (step + 1))
+    idx = [splitmix64(key ^ (s * 0xD6E8FEB86659FD93 & (1 << 64) - 1)) % len(targ) for s in range(batch)]
+    return mo.gradient(mo.params_of(net), feats[idx], targ[idx])[1]
+
+
+@pytest.mark.parametrize("steps", [1, 2, 15, 20, 25])
+def test_reported_losses_are_those_of_the_first_and_last_steps(samples, steps):
+    """loss_first and loss_last are the mean losses of the first and the last
+    tenth of the steps: each step's loss is that of the weights before it on
+    the samples it draws (a run of one step has no last tenth of its own)."""
+    tr, feats, targ, _, _ = samples
+    kw = dict(batch=300, lr=3e-3, seed=9)
+    window = max(1, steps // 10)
+
+    def loss(i):
+        net, _ = tr.fit(steps=i, **kw) if i else tr.fit(steps=1, **dict(kw, lr=1e-30))
+        return batch_loss(net, feats, targ, kw["seed"], i, kw["batch"])
+
+    _, rep = tr.fit(steps=steps, **kw)
+    first = np.mean([loss(i) for i in range(window)])
+    assert abs(rep["loss_first"] - first) <= 1e-4 * first
+    if steps == 1:
+        assert rep["loss_last"] == 0.0
+        return
+    last = np.mean([loss(i) for i in range(steps - window, steps)])
+    assert abs(rep["loss_last"] - last) <= 1e-4 * last
+
+
+@pytest.mark.parametrize("q", [19, 27])
+@pytest.mark.parametrize("nx", [32, 16], ids=["tile32", "tile16"])
+@pytest.mark.parametrize("z_chunk", [1, 2, 5, 12])
+def test_fused_network_over_several_planes_of_an_item(samples, q, nx, z_chunk):
+    """Items of one and of several planes: the network inside the step kernel
+    reuses its tensor memory, operands and barriers from plane to plane and
+    hands each plane's range check to the next; the bits of the separate
+    kernels."""
+    _, feats, targ, _, _ = samples
+    net = random_net(feats, targ, seed=12, scale=0.5)
+    kw = dict(tile=(nx, 8, 2), pop_buffers=1)
+    with Cavity(q, nx, 16, 24, 300.0, 0.05, z_chunk=z_chunk, **kw) as a, \
+            Cavity(q, nx, 16, 24, 300.0, 0.05, z_chunk=24, **kw) as b:
+        for c in (a, b):
+            c.init_regions()
+            c.set_closure(net)
+        b.closure_fused(False)
+        for c in (a, b):
+            c.step(7)
+            c.synchronize()
+        assert a.info()["z_chunk"] == z_chunk and a.info()["tile_x"] == nx
+        da, db = a.closure_dtau(), b.closure_dtau()
+        assert np.count_nonzero(db) > 0 and np.count_nonzero(db == 0.0) > 0  # in and out of the training range
+        assert np.array_equal(bits(da), bits(db))
+        assert np.array_equal(bits(a.read()), bits(b.read()))
+
+
+@pytest.mark.parametrize("q,nx", [(19, 256), (27, 264)])
+@pytest.mark.parametrize("fused", [True, False])
+def test_closure_on_a_grid_that_ends_in_quarter_chunks(samples, q, nx, fused):
+    """Both evaluations on a grid of two waves (the closure's steps take their
+    z-chunks from the same rule as the plain ones): the bits of short uniform
+    chunks."""
+    _, feats, targ, _, _ = samples
+    net = random_net(feats, targ, seed=13, scale=0.5)
+    shape, kw = (nx, 256, 72), dict(tile=(32, 8, 2), pop_buffers=1)
+    assert -(-nx // 32) * 32 * -(-72 // 16) * 8 >= 2 * 148 * 24  # z_chunks tapers chunks of 16 planes
+    with Cavity(q, *shape, 300.0, 0.05, z_chunk=16, **kw) as a, Cavity(q, *shape, 300.0, 0.05, z_chunk=6, **kw) as b:
+        for c in (a, b):
+            c.init_regions()
+            c.perturb_velocity(1e-3, 3)
+            c.set_closure(net)
+            c.closure_fused(fused)
+            c.step(4)
+            c.synchronize()
+        assert np.array_equal(bits(a.closure_dtau()), bits(b.closure_dtau()))
+        assert np.array_equal(bits(a.read()), bits(b.read()))
