@@ -253,17 +253,21 @@ bool pick_launcher(int Q, int tx, int ty, int stages, int npb, int storage, unsi
 
 // Default kernel shape of a mesh: the tile width and z-chunk with the least
 // predicted time per step.  A plane of the march costs every SM
-// max(floor, base + per_cta * n) us with n CTAs on it (D3Q19, FP32; D3Q27 takes
-// 1.25 times as long in every term, so the choice is the same): the floor is
-// the chain of one plane -- copy, reconstruction, barrier, update -- that a
-// lone CTA waits out, per_cta the issue slots of a tile.  A grid with a
-// tapered end (z_chunks) is charged for the planes its CTAs visit and half a
-// chunk of draining.  Tiles with more than half of their lanes outside the
-// mesh are left out.  Over 38 meshes from 32x16x24 to 192^3 the choice is
-// within 15% of the fastest (tile, z-chunk), 3% on average.  D3Q19, us per
-// step, the former rule (widest tile that divides nx, chunks of 9 or more,
-// former kernels) -> this one: 32x16x24 20.6 -> 3.6, 8x64x64 29.1 -> 4.5,
-// 64^3 24.0 -> 8.8, 88x96x104 33.2 -> 23.2, 296x264x248 667 -> 304.
+// max(floor, base + per_cta * n) us with n CTAs on it: the floor is the chain
+// of one plane -- copy, reconstruction, barrier, update -- that a lone CTA
+// waits out, per_cta the issue slots of a tile.  A grid with a tapered end
+// (z_chunks) is charged for the planes its CTAs visit and half a chunk of
+// draining.  Tiles with more than half of their lanes outside the mesh are
+// left out.  The constants are those of D3Q19 in FP32 without function
+// objects; the other kernels take longer in every term, and the choice serves
+// them as well: against lbm_autotune's, over ten meshes from 32x16x24 to
+// 296x264x248, D3Q19 and D3Q27 each in FP32, in FP16, with S/SMean/k/kMean and
+// with all function objects and FP64 means, it is 3-6% slower on average and
+// at most 20% (the last set on the smallest mesh; else 17%, on 88x96x104).
+// D3Q19, us per step, the former rule (widest tile that divides nx, chunks of
+// 9 or more, former kernels) -> this one: 32x16x24 20.6 -> 3.5, 8x64x64 29.1
+// -> 4.4, 64^3 24.0 -> 8.7, 88x96x104 33.5 -> 23.1, 296x264x248 731 -> 308;
+// of 460 meshes, storage formats and function objects none is slower.
 void default_tiling(int64_t nx, int64_t ny, int64_t nz, int only_tx, bool narrow, int &tx, int &zc)
 {
     struct Tile {

@@ -68,8 +68,10 @@ __device__ __forceinline__ void cta_sync()
 // and is visible.  Both do nothing in a kernel launched without the attribute.
 // Letting the next grid start earlier costs more than it hides: its CTAs then
 // land where slots are free and leave the SMs unevenly loaded (64^3 D3Q19, us
-// per step: no overlap 9.4, from the start of the item 11.1, from its last
-// plane 9.9, after it 8.9).
+// per step: no overlap 9.75, from the start of the item 11.1, from its last
+// plane 9.9, after it 9.13).  With the current kernels, no overlap / after the
+// item: D3Q19 64^3 9.07 / 8.63, D3Q27 64^3 10.8 / 10.3, D3Q27 8^3 4.4 / 3.9,
+// D3Q27 72x40x40 with S/SMean/k/kMean 12.3 / 9.4, D3Q27 256^3 the same.
 __device__ __forceinline__ void let_next_grid_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_previous_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

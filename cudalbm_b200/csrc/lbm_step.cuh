@@ -180,9 +180,11 @@ static_assert(offsetof(StepParamsF32, fault) == offsetof(StepParamsF64Means, fau
 // With at least two waves of work on the GPU (24 warps per SM are resident)
 // the end of z, 3/4 to 7/4 of a chunk, is therefore cut into quarter chunks;
 // CTAs start in the order of their chunk, so these fill the end of the grid.
-// 256^3, us per step, best uniform chunk (19) / 32 + quarters: D3Q27 334.1 /
-// 325.5, D3Q19 250.4 / 246.8, D3Q19 FP16 245.7 / 239.8; with 26 + quarters
-// D3Q27 with S/SMean/k/kMean 486.7 / 484.1.
+// 256^3, us per step with the best uniform chunk / the best chunk with
+// quarters: D3Q27 328.0 (22 planes) / 317.3 (37), D3Q19 at 4 CTAs/SM 244.8 (19)
+// / 241.9 (20), its FP16 storage 241.5 (19) / 235.9 (37), D3Q27 with
+// S/SMean/k/kMean 489.5 (14) / 488.9 (16); at one chunk of 32 planes 338.9 /
+// 321.2, 271.4 / 256.2, 253.4 / 236.4 and 521.9 / 498.1.
 struct ZChunks {
     int zc, nbig, zc2, count;
 };

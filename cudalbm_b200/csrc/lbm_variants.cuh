@@ -57,8 +57,16 @@ template <int Q, int TX, int TY, int NS, int NPB, int MINB, typename ST, int FO>
 void pick_means(Launcher &l, int mean_bits)
 {
     if (mean_bits == 64) {
-        // FP64 old means of all moments: 20 registers more are worth a CTA
-        // (256^3, all five: 1126 us per step at 3 CTAs/SM, 1058 at 2)
+        // FP64 old means of all moments: with the six of SMean 20 registers
+        // more are worth a CTA.  us per step of 32-wide tiles at 3 / 2 CTAs
+        // per SM, best of the z-chunks 2 to 26, all five function objects:
+        // D3Q27 64^3 17.2 / 16.3, 136x120x128 154.6 / 152.1, 256^3 1043 /
+        // 1039, D3Q19 256^3 1049 / 1030, D3Q27 256^3 in FP16 storage 925 /
+        // 944; at the default chunk of 256^3 2 CTAs take 0.94-0.96 of the
+        // time.  Sets without SMean gain on small meshes and lose on large
+        // ones (momentsMean alone, D3Q27: 64^3 14.3 / 13.1, 96^3 39.8 / 46.2,
+        // 256^3 685 / 748, in FP16 storage 611 / 701).  16- and 8-wide tiles
+        // run the same within 3%.
         constexpr int MB = FO == 3 && MINB > 2 ? 2 : MINB;
         l.fn = kernel_fn<Q, TX, TY, NS, FO, double, false, NPB, MB, ST>();
         l.fn_mon = kernel_fn<Q, TX, TY, NS, FO, double, true, NPB, MB, ST>();
