@@ -251,14 +251,29 @@ bool pick_launcher(int Q, int tx, int ty, int stages, int npb, int storage, unsi
                    : lbm::pick_q27_f32(tx, ty, stages, npb, fo, mean_bits, out);
 }
 
+// Predicted time per step, in us, of a mesh of nz planes of `tiles` tiles in
+// chunks z.  A plane of the march costs every SM max(floor, base + per_cta * n)
+// us with n CTAs on it: the floor is the chain of one plane -- copy,
+// reconstruction, barrier, update -- that a lone CTA waits out, per_cta the
+// issue slots of a tile.  A grid with a tapered end (z_chunks) is charged for
+// the planes its CTAs visit and half a chunk of draining.
+struct TileCost {
+    int tx;
+    double floor, base, per_cta;
+};
+constexpr TileCost kTileCosts[] = {{32, 1.1, 0.33, 0.55}, {16, 1.1, 0.6, 0.29}, {8, 1.1, 0.6, 0.21}};
+
+double predicted_us(const TileCost &t, int64_t nz, int64_t tiles, const lbm::ZChunks &z)
+{
+    constexpr double kSms = 148.0;
+    if (z.zc2 != z.zc)
+        return t.per_cta * double(tiles) * double(nz + 2 * z.count) / kSms + 0.5 * t.base * (z.zc + 2);
+    return (z.zc + 2) * std::max(t.floor, t.base + t.per_cta * std::ceil(double(tiles) * z.count / kSms));
+}
+
 // Default kernel shape of a mesh: the tile width and z-chunk with the least
-// predicted time per step.  A plane of the march costs every SM
-// max(floor, base + per_cta * n) us with n CTAs on it: the floor is the chain
-// of one plane -- copy, reconstruction, barrier, update -- that a lone CTA
-// waits out, per_cta the issue slots of a tile.  A grid with a tapered end
-// (z_chunks) is charged for the planes its CTAs visit and half a chunk of
-// draining.  Tiles with more than half of their lanes outside the mesh are
-// left out.  The constants are those of D3Q19 in FP32 without function
+// predicted time per step.  Tiles with more than half of their lanes outside
+// the mesh are left out.  The constants are those of D3Q19 in FP32 without function
 // objects; the other kernels take longer in every term, and the choice serves
 // them as well: against lbm_autotune's, over ten meshes from 32x16x24 to
 // 296x264x248, D3Q19 and D3Q27 each in FP32, in FP16, with S/SMean/k/kMean and
@@ -270,15 +285,9 @@ bool pick_launcher(int Q, int tx, int ty, int stages, int npb, int storage, unsi
 // of 460 meshes, storage formats and function objects none is slower.
 void default_tiling(int64_t nx, int64_t ny, int64_t nz, int only_tx, bool narrow, int &tx, int &zc)
 {
-    struct Tile {
-        int tx;
-        double floor, base, per_cta;
-    };
-    constexpr Tile kTiles[] = {{32, 1.1, 0.33, 0.55}, {16, 1.1, 0.6, 0.29}, {8, 1.1, 0.6, 0.21}};
-    constexpr double kSms = 148.0;
     double best = 1e300;
     zc = int((nz + 65534) / 65535);  // the grid's z limit, for meshes longer than any chunk below allows
-    for (const Tile &t : kTiles) {
+    for (const TileCost &t : kTileCosts) {
         if (only_tx ? t.tx != only_tx : (t.tx == 8 && !narrow) || (t.tx > 8 && nx <= t.tx / 2 && (narrow || t.tx > 16)))
             continue;
         const int64_t tiles = ((nx + t.tx - 1) / t.tx) * ((ny + 7) / 8);
@@ -288,11 +297,7 @@ void default_tiling(int64_t nx, int64_t ny, int64_t nz, int only_tx, bool narrow
             const lbm::ZChunks z = lbm::z_chunks(nz, c, tiles, t.tx * 8 / 32);
             if (z.count > 65535)
                 continue;
-            double us;
-            if (z.zc2 != z.zc)
-                us = t.per_cta * double(tiles) * double(nz + 2 * z.count) / kSms + 0.5 * t.base * (c + 2);
-            else
-                us = (c + 2) * std::max(t.floor, t.base + t.per_cta * std::ceil(double(tiles) * z.count / kSms));
+            const double us = predicted_us(t, nz, tiles, z);
             if (us < best) {
                 best = us;
                 tx = t.tx;
@@ -1795,16 +1800,13 @@ lbm_status lbm_autotune(lbm_handle *h, int32_t trial_steps, lbm_tuning *out)
         // (such a chunk re-reads two planes for every 2-4 it updates)
         const int64_t tiles = ((h->cfg.nx + v.tx - 1) / v.tx) * ((h->cfg.ny + v.ty - 1) / v.ty);
         const bool small = tiles * ((h->cfg.nz + 7) / 8) < 4 * 148 * 3;
-        // Candidates: powers of two; where the grid's end is tapered
-        // (z_chunks), lengths between them, since any such chunk may be the
-        // best by a few percent; where it is not, those whose grid is close
-        // to a whole number of waves of resident CTAs (k waves for k = 1..12):
-        // the last wave of a grid 9.2 waves long runs the GPU at a fifth of
-        // its CTA slots.  Lengths between the powers of two on every grid made
-        // the call 1.5 times as long (78 lattices, meshes and field sets; 1.9
-        // times on the small ones) for steps that were no faster (1.0005).
-        // Chunks need not divide nz (the last is shorter).
-        std::vector<int> zcs = {2, 4, 8, 16, 32, 64};
+        // Candidates: a ladder of lengths, finer above 16 where such a chunk
+        // tapers the grid's end (z_chunks); where none does, those whose grid
+        // is close to a whole number of waves of resident CTAs (k waves for
+        // k = 1..12): the last wave of a grid 9.2 waves long runs the GPU at a
+        // fifth of its CTA slots.  Chunks need not divide nz (the last is
+        // shorter).
+        std::vector<int> zcs = {1, 2, 3, 4, 6, 8, 11, 16, 32, 64};
         for (int zc : {20, 26, 37, 43, 52})
             if (const lbm::ZChunks z = lbm::z_chunks(h->cfg.nz, zc, tiles, v.tx * v.ty / 32); z.zc2 != z.zc)
                 zcs.push_back(zc);
@@ -1826,10 +1828,33 @@ lbm_status lbm_autotune(lbm_handle *h, int32_t trial_steps, lbm_tuning *out)
                 }
             }
         }
+        // Lengths predicted to take more than 1.3 times the best of them are
+        // not timed, and a variant's kernels are set up once: over 138 drawn
+        // meshes, storage formats and function objects a call takes 0.35 of
+        // the time of one that sets up and times each length of the ladder
+        // (10 to 50 ms on meshes of up to two million nodes), and the steps
+        // are as fast (0.9996).
+        const TileCost &cost = *std::find_if(std::begin(kTileCosts), std::end(kTileCosts),
+                                             [&](const TileCost &t) { return t.tx == v.tx; });
+        std::vector<std::pair<int, double>> timed;
+        double least = 1e300;
         for (int zc : zcs) {
             if (zc > h->cfg.nz || (zc < 8 && !small))
                 continue;
-            lbm_status s = apply_variant(h, v.tx, v.ty, v.stages, v.npb, zc);
+            timed.emplace_back(zc, predicted_us(cost, h->cfg.nz, tiles,
+                                                lbm::z_chunks(h->cfg.nz, zc, tiles, v.tx * v.ty / 32)));
+            least = std::min(least, timed.back().second);
+        }
+        bool placed = false;  // the handle has this variant's kernels and tensor maps
+        for (const auto &[zc, predicted] : timed) {
+            if (predicted > 1.3 * least)
+                continue;
+            lbm_status s = LBM_OK;
+            if (placed)
+                h->zc = zc;
+            else
+                s = apply_variant(h, v.tx, v.ty, v.stages, v.npb, zc);
+            placed = true;
             if (s != LBM_OK) {
                 release();
                 return s;

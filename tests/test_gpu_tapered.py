@@ -103,9 +103,9 @@ def test_streamed_middle_steps(q, nx, storage, fo):
 
 
 @pytest.mark.parametrize("shape,most", [((64, 64, 64), 54), ((72, 40, 40), 42), ((8, 64, 64), 7)])
-def test_autotune_tries_few_chunks_where_none_tapers(shape, most):
-    """The lengths between the powers of two are timed on tapered grids only:
-    on a small mesh a call takes no longer than powers of two and whole waves."""
+def test_autotune_times_few_chunks_on_small_meshes(shape, most):
+    """Of the chunk lengths only those are timed that may be the fastest: on a
+    small mesh no more of them than powers of two and whole waves."""
     assert not tapers(*shape, 8, 16) and not tapers(*shape, 32, 16)
     with Cavity(19, *shape, 400.0, 0.05) as c:
         c.init_regions()
