@@ -847,9 +847,12 @@ lbm_status lbm_create(const lbm_config *cfg, lbm_handle **out)
     default_tiling(c.nx, c.ny, c.nz, named ? tx : 0, h->storage == 0, tx, zc);
     if (c.z_chunk) zc = c.z_chunk;
     const unsigned fo = c.function_objects;
-    // D3Q19 without function objects fits four CTAs per SM at 64 registers;
-    // grids with more than three per SM gain (256^3 258.6 -> 248.3 us per
-    // step, FP16 262 -> 243), smaller ones have no use for the fourth
+    // D3Q19 without function objects fits four CTAs per SM at 64 registers.
+    // Grids with more than three per SM gain, smaller ones have no use for the
+    // fourth.  us per step at 3 / 4 CTAs per SM: 256^3 (2560 CTAs) 258.5 /
+    // 243.8, FP16 244.6 / 237.3, 128^3 (1024) 44.3 / 41.6, 64^3 in 2-plane
+    // chunks (512) 10.0 / 8.4, in 4-plane ones (256) 8.7 / 8.7; an exception
+    // is 96^3 in 4-plane chunks (864) 19.8 / 20.8.
     const int64_t ctas = ((c.nx + 31) / 32) * ((c.ny + 7) / 8) * ((c.nz + std::max(zc, 1) - 1) / std::max(zc, 1));
     const bool four = !named && h->Q == 19 && !fo && tx == 32 && ctas > 3 * 148;
     const int npb = c.pop_buffers ? c.pop_buffers : (four ? 4 : 1);
